@@ -14,7 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libedge_b200.so")
-SOURCES = ["solver.cu"]
+OBJDIR = os.path.join(HERE, "_build")
+SOURCES = ["solver.cu", "fields.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -25,28 +26,57 @@ def nvcc_path():
     raise RuntimeError("nvcc not found")
 
 
-def _stale():
-    if not os.path.exists(LIB):
+def _headers():
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cu")] + \
+        [os.path.join(ROOT, "include", "edge_b200.h")]
+
+
+def _older(target, deps):
+    """True when target is missing or older than one of deps."""
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "edge_b200.h")]
+    t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def _stale():
+    return _older(LIB, [os.path.join(CSRC, s) for s in SOURCES] + _headers())
+
+
 def build(force=False, verbose=False, extra=()):
+    """Compile every stale source to an object (in parallel, each with parallel code
+    generation) and link the library."""
     if not force and not _stale():
         return LIB
-    cmd = [nvcc_path(), "-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC", "-shared",
-           "-cudart", "static", "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"),
-           *extra, "-o", LIB + ".tmp", *[os.path.join(CSRC, s) for s in SOURCES]]
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    r = subprocess.run(cmd, capture_output=True, text=True)
+    os.makedirs(OBJDIR, exist_ok=True)
+    flags = ["-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC", "-cudart", "static",
+             "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include")]
+    jobs, objs = [], []
+    for src in SOURCES:
+        path, obj = os.path.join(CSRC, src), os.path.join(OBJDIR, src + ".o")
+        objs.append(obj)
+        if force or extra or _older(obj, [path] + _headers()):
+            cmd = [nvcc_path(), "-c", *flags, "--split-compile", "0", *extra, "-o", obj + ".tmp", path]
+            if verbose:
+                print(" ".join(cmd), flush=True)
+            jobs.append((obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    failed = False
+    for obj, job in jobs:
+        out, _ = job.communicate()
+        if job.returncode != 0:
+            failed = True
+            sys.stderr.write(out)
+        else:
+            os.replace(obj + ".tmp", obj)
+            if verbose and out:
+                sys.stderr.write(out)
+    if failed:
+        raise RuntimeError("nvcc failed building libedge_b200.so")
+    r = subprocess.run([nvcc_path(), *ARCH, "-shared", "-cudart", "static", "-o", LIB + ".tmp", *objs],
+                       capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError("nvcc failed building libedge_b200.so")
-    if verbose and r.stderr:
-        sys.stderr.write(r.stderr)
+        raise RuntimeError("nvcc failed linking libedge_b200.so")
     os.replace(LIB + ".tmp", LIB)
     return LIB
 

@@ -551,97 +551,6 @@ __global__ void __launch_bounds__(BT) k_batch_pcg(const BatchDesc* D, int nprob,
   }
 }
 
-// ------------------------------------------------------------------ OC updates of many problems
-// One block per problem (taken from a queue like the solve): the OC update of k_oc_prep,
-// k_oc_floor, k_oc_pass and k_oc_final (TopOpt/_cuda.py:242-280) with every sum a block sum in a
-// fixed order and the bisection tree walked by every thread alike; at most 50 passes of
-// OC_DEPTH bisection steps (the per-problem loop's bound of 200 steps).
-struct BatchOcDesc {
-  long long n;
-  const double* rho;
-  const double* dr;
-  double* ocp;
-  double* rho_new;
-  double A, vol, vf;
-};
-
-template <int BT>
-__global__ void __launch_bounds__(BT) k_batch_oc(const BatchOcDesc* D, int nprob, unsigned* queue, double move,
-                                                 double* lam_out, int* steps_out) {
-  using TM = Team<1>;
-  __shared__ double sh[34];
-  __shared__ int s_idx;
-  for (;;) {
-    if (threadIdx.x == 0) s_idx = (int)atomicAdd(queue, 1u);
-    __syncthreads();
-    const int idx = s_idx;
-    __syncthreads();
-    if (idx >= nprob) return;
-    const BatchOcDesc d = D[idx];
-    const long long n = d.n;
-    double acc = 0.0;
-    for (long long i = threadIdx.x; i < n; i += BT) {
-      double v = d.rho[i] * sqrt(fmax(-d.dr[i] / d.A, 0.0));
-      if (isnan(v)) v = 0.0;
-      acc += fabs(v);
-      d.ocp[i] = v;
-    }
-    const bool allzero = TM::sum(acc, sh) == 0.0;
-    for (long long i = threadIdx.x; i < n; i += BT) d.ocp[i] = fmax(1e-12, allzero ? 1e-3 : d.ocp[i]);
-    __syncthreads();
-    double l1 = 1e-9, l2 = 1e9, last = 0.5 * (l1 + l2);
-    int steps = 0;
-    bool done = false;
-    const int max_pass = (200 + OC_DEPTH - 1) / OC_DEPTH;
-    for (int pass = 0; pass < max_pass && !done; ++pass) {
-      double lam[OC_NODES];
-      {
-        double L1[OC_NODES], L2[OC_NODES];
-        L1[0] = l1;
-        L2[0] = l2;
-        for (int t = 0; t < OC_NODES; ++t) {
-          lam[t] = 0.5 * (L1[t] + L2[t]);
-          if (2 * t + 2 < OC_NODES) {
-            L1[2 * t + 1] = L1[t];
-            L2[2 * t + 1] = lam[t];
-            L1[2 * t + 2] = lam[t];
-            L2[2 * t + 2] = L2[t];
-          }
-        }
-      }
-      double a[OC_NODES];
-      for (int t = 0; t < OC_NODES; ++t) a[t] = 0.0;
-      for (long long i = threadIdx.x; i < n; i += BT) {
-        const double r = d.rho[i], o = d.ocp[i];
-        for (int t = 0; t < OC_NODES; ++t) a[t] += oc_rho(r, o, lam[t], move) * d.A;
-      }
-      double sums[OC_NODES];
-      for (int t = 0; t < OC_NODES; ++t) sums[t] = TM::sum(a[t], sh);
-      int t = 0;
-      for (int dd = 0; dd < OC_DEPTH; ++dd) {
-        if (!((l2 - l1) / (l2 + l1) > 1e-4)) {
-          done = true;
-          break;
-        }
-        const double mid = 0.5 * (l1 + l2);
-        const bool valid = (sums[t] / d.vol <= d.vf);
-        if (valid) l2 = mid;
-        else l1 = mid;
-        last = mid;
-        steps += 1;
-        t = 2 * t + (valid ? 1 : 2);
-      }
-      if (!((l2 - l1) / (l2 + l1) > 1e-4)) done = true;
-    }
-    for (long long i = threadIdx.x; i < n; i += BT) d.rho_new[i] = oc_rho(d.rho[i], d.ocp[i], last, move);
-    if (threadIdx.x == 0) {
-      lam_out[idx] = last;
-      steps_out[idx] = steps;
-    }
-    __syncthreads();
-  }
-}
-
 // User node order (reference numbering of the real nx_r x ny_r grid) <-> slots of a grid that
 // may be larger (padded): slots outside the real grid are zero.
 __global__ void k_user_to_slots_pad(const Geo g, int nxr, int nyr, const double* __restrict__ user,

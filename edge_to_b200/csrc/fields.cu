@@ -1,0 +1,541 @@
+// Element-wise passes on arrays in the user's layout (declared in fields.cuh).
+#include "fields.cuh"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <atomic>
+
+namespace edge {
+
+// ------------------------------------------------------------------ OC design update
+// The OC update of TopOpt/_cuda.py:242-280: ocP = max(1e-12, rho sqrt(max(-dr / A, 0))) (1e-3
+// everywhere when all are zero, MaterialModels.py:75-88), the bisection of the multiplier in
+// [1e-9, 1e9] until (l2 - l1) / (l2 + l1) <= 1e-4 (at most 200 steps), rho_new at the last
+// multiplier tried and sum((rho_new - rho)^2).
+//
+// What bounds it: the bisection is a serial chain of about 45 decisions "is sum(rho_new(mid)) A
+// <= vf vol", each a sum over all elements.  The sum does not increase with the multiplier, so a
+// decision is known without a sum when mid lies outside the interval (a, b) between the
+// largest multiplier seen to be infeasible and the smallest seen to be feasible.  A pass
+// therefore evaluates OC_CAND multipliers spread evenly in log over (a, b), which takes the
+// 16th root of its ratio: four passes from 1e18 to 1.0007; then the few midpoints that still
+// fall inside (a, b) are evaluated as a tree, four deep per pass, and walked exactly as the
+// sequential bisection would, so the multiplier used is a midpoint of that bisection, decided
+// on an evaluated sum or by monotonicity.  A pass ends in the block that finishes last: it sums
+// the blocks' partials, moves the bracket and leaves the next candidates; no block waits for
+// another.  The number of passes is fixed (OC_PASSES), those after the end return at once, so
+// neither a host read nor a graph condition is needed between them.
+//
+// A candidate costs one multiply by the reciprocal multiplier, the two bounds and one FMA per
+// element (rho_new itself is divided, as the reference does).
+constexpr int OC_PASSES = 6;  // four spread, one of the tree, one more when the first only finds all ocP zero
+
+// The upper ends of the bracket while every midpoint is feasible: l2[k + 1] = (1e-9 + l2[k]) / 2,
+// all of them far from the end of the bisection (the bracket stays wider than 4 to 1).  Most
+// updates begin with about 30 such steps; a chain of dependent FP64 operations, walked here by
+// bisection on the step number instead.
+constexpr int OC_CHAIN = 57;
+struct OcChain {
+  double l2[OC_CHAIN + 1];
+};
+constexpr OcChain make_oc_chain() {
+  OcChain c{};
+  c.l2[0] = 1e9;
+  for (int k = 0; k < OC_CHAIN; ++k) c.l2[k + 1] = 0.5 * (1e-9 + c.l2[k]);
+  return c;
+}
+__constant__ OcChain c_oc_chain = make_oc_chain();
+static_assert(make_oc_chain().l2[OC_CHAIN] > 4e-9, "the chain ends before the bracket closes");
+
+// Bisection bracket; mids outside (a, b) are decided by monotonicity.
+struct OcBis {
+  double l1, l2, last, a, b;
+  int steps;
+  // (l2 - l1) / (l2 + l1) > 1e-4; the division only where rounding could decide it
+  EDGE_D bool open() const {
+    const double d = l2 - l1, s = l2 + l1;
+    bool o = d > 1.0000001e-4 * s;
+    if (!o && d > 0.9999999e-4 * s) o = d / s > 1e-4;
+    return o && steps < 200;
+  }
+  EDGE_D void take(bool valid) {
+    const double mid = 0.5 * (l1 + l2);
+    if (valid) l2 = mid;
+    else l1 = mid;
+    last = mid;
+    ++steps;
+  }
+  // decides midpoints while they lie outside (a, b); true: the bisection has ended
+  EDGE_D bool advance() {
+    if (steps < OC_CHAIN && l1 == 1e-9 && l2 == c_oc_chain.l2[steps]) {
+      // every step so far was feasible: the last k with c_oc_chain.l2[k] >= b, by halving
+      int k = steps;
+#pragma unroll
+      for (int h = 32; h >= 1; h >>= 1)
+        if (k + h <= OC_CHAIN && c_oc_chain.l2[k + h] >= b) k += h;
+      if (k > steps) {
+        last = l2 = c_oc_chain.l2[k];
+        steps = k;
+      }
+    }
+    while (open()) {
+      const double mid = 0.5 * (l1 + l2);
+      if (mid >= b) take(true);
+      else if (mid <= a) take(false);
+      else return false;
+    }
+    return true;
+  }
+  EDGE_D void decide(bool valid) {  // outcome of an evaluated midpoint
+    const double mid = 0.5 * (l1 + l2);
+    if (valid) b = mid;
+    else a = mid;
+    take(valid);
+  }
+};
+
+// Sum of v[0..15] over the block's threads into out[0..15] (shared memory, valid after the
+// block's next barrier); sw: 16 doubles per warp of scratch.  A warp folds the 16 values across
+// its lanes (each exchange halves the values a lane still carries): 16 exchanges for 16 sums.
+EDGE_D void block_sum16(double v[16], double* sw, double* out) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int h = 8; h >= 1; h >>= 1) {
+    const bool up = lane & h;
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+      if (t < h) {
+        const double keep = up ? v[t + h] : v[t], give = up ? v[t] : v[t + h];
+        v[t] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+      }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+  if (lane < 16) sw[wid * 16 + lane] = v[0];  // lane t of every warp holds the warp's sum of value t
+  __syncthreads();
+  if (wid < 16) {  // warp t finishes value t (at least 16 warps)
+    double s = lane < nw ? sw[lane * 16 + wid] : 0.0;
+    s = warp_sum(s);
+    if (lane == 0) out[wid] = s;
+  }
+}
+
+// Where a pass evaluates need not be exact, only ascending inside (ca, cb): FP32 logarithm and
+// power (the ratio is at least 1.002, its 16th root 1000 FP32 roundings above 1).
+EDGE_D double oc_spread(double ca, double cb, int t) {
+  const float l = log2f(__fdividef((float)cb, (float)ca));
+  const double lam = ca * (double)exp2f(l * ((t + 1) * 0.0625f));
+  return lam < cb ? lam : cb;
+}
+EDGE_D double oc_value(double r, double o, double lam, double move) {
+  const double xU = fmin(fmax(r + move, 0.0), 1.0);
+  const double xL = fmin(fmax(r - move, 0.0), 1.0);
+  return fmax(0.0, fmax(xL, fmin(1.0, fmin(xU, o / lam))));
+}
+
+// The interval of multipliers not yet known to be feasible or infeasible is wide: spread.
+EDGE_D bool oc_wide(const OcBis& B) { return B.b > 1.002 * B.a; }
+// sum / vol <= vf; the division only where rounding could decide it.
+EDGE_D bool oc_feasible(double sum, double vol, double vf) {
+  const double t = vf * vol;
+  if (vol > 0.0 && sum < t * 0.999999999) return true;
+  if (vol > 0.0 && sum > t * 1.000000001 && t > 0.0) return false;
+  return sum / vol <= vf;
+}
+// Moves the bracket by the outcomes of one pass (bit t of ok: candidate t is feasible); true: the
+// bisection has ended.  The bisection itself only starts once (a, b) is narrow.
+EDGE_D bool oc_move(OcBis& B, bool spread, unsigned ok, const double* lam) {
+  if (spread) {
+    // the candidates ascend: the first feasible one bounds (a, b) above, the one before it below
+    const int t = __ffs(ok) - 1;
+    if (t >= 0) B.b = lam[t];
+    if (t != 0) B.a = lam[(t > 0 ? t : OC_CAND) - 1];
+    return oc_wide(B) ? false : B.advance();
+  }
+  bool done = false;
+  int t = 0;
+  for (int d = 0; d < 4 && !done; ++d) {
+    const bool valid = (ok >> t) & 1;
+    B.decide(valid);
+    done = B.advance();
+    t = 2 * t + (valid ? 1 : 2);
+  }
+  return done;
+}
+// Candidate t of the pass after bracket B: spread over (a, b) while that is wide, then the
+// heap-ordered tree of undecided midpoints (the bits of the node give the outcomes on its path).
+EDGE_D double oc_candidate(OcBis C, int t) {
+  if (oc_wide(C)) return oc_spread(C.a, C.b, t);
+  const int node = t + 1;
+  bool end = false;
+  for (int d = 30 - __clz(node); d >= 0 && !end; --d) {
+    C.decide(!((node >> d) & 1));  // left child: feasible
+    end = C.advance();
+  }
+  return 0.5 * (C.l1 + C.l2);
+}
+// (a, b) starts at the bracket's ends: every midpoint lies strictly between them
+EDGE_D OcBis oc_start() { return OcBis{1e-9, 1e9, 0.5 * (1e-9 + 1e9), 1e-9, 1e9, 0}; }
+EDGE_D double oc_raw(double r, double dr, double A) {
+  const double o = r * sqrt(fmax(-dr / A, 0.0));
+  return isnan(o) ? 0.0 : o;
+}
+// The candidates' design values of one element (move limits xl, xu; o not NaN: at least 1e-12)
+// times A, added to v.
+EDGE_D double oc_clip01(double x) {  // fmin(fmax(x, 0), 1): 0 for a NaN
+  x = x > 0.0 ? x : 0.0;
+  return x < 1.0 ? x : 1.0;
+}
+EDGE_D void oc_eval(double r, double o, double move, double A, const double* ilam, double v[16]) {
+  const double xu = oc_clip01(r + move), xl = oc_clip01(r - move);
+#pragma unroll
+  for (int t = 0; t < OC_CAND; ++t) {
+    double x = o * ilam[t];
+    x = x < xu ? x : xu;
+    x = x > xl ? x : xl;
+    v[t] = fma(x, A, v[t]);
+  }
+}
+
+// One pass.  PASS 0 computes ocP as well; PASS 2 (the third pass and later) is launched so that its
+// blocks may start while the pass before is still finishing: rho and ocP are settled by then
+// (the pass before let its dependents start after pass 0 had completed), so each thread fetches
+// its first elements before it waits for that pass's candidates.
+template <int PASS>
+__global__ void __launch_bounds__(OC_THREADS)
+k_oc_bisect(long long n, const double* __restrict__ rho, const double* __restrict__ dr, double A, double vol, double vf,
+            double move, double* __restrict__ ocp, double* part, unsigned* ticket, OcState* st) {
+  constexpr int PRE = 2;
+  __shared__ double sw[16 * 16];
+  __shared__ double ssum[16];
+  __shared__ double slam[16], silam[16];
+  __shared__ bool am_last;
+  __shared__ OcBis sB;
+  const long long i0 = blockIdx.x * (long long)OC_THREADS + threadIdx.x, T = (long long)gridDim.x * OC_THREADS;
+  double pr[PRE], po[PRE];
+  if constexpr (PASS == 2) {
+#pragma unroll
+    for (int q = 0; q < PRE; ++q) {
+      const long long i = i0 + q * T < n ? i0 + q * T : n - 1;
+      pr[q] = rho[i];
+      po[q] = ocp[i];
+    }
+  }
+  EDGE_PDL_ENTRY();
+  if (PASS != 0 && st->done) return;
+  const bool allz = PASS == 0 ? false : st->allzero != 0;
+  if (threadIdx.x < OC_CAND) {
+    const double lam = PASS == 0 ? oc_spread(1e-9, 1e9, threadIdx.x) : st->lam[threadIdx.x];
+    slam[threadIdx.x] = lam;
+    silam[threadIdx.x] = 1.0 / lam;
+  }
+  __syncthreads();
+  double v[16];
+#pragma unroll
+  for (int t = 0; t < 16; ++t) v[t] = 0.0;
+  bool any = false;
+  long long i = i0;
+  if constexpr (PASS == 2) {
+#pragma unroll
+    for (int q = 0; q < PRE; ++q)
+      if (i0 + q * T < n) oc_eval(pr[q], allz ? 1e-3 : po[q], move, A, silam, v);
+    i += PRE * T;
+  }
+  constexpr int U = 4;  // elements fetched together
+  for (; i < n; i += U * T) {
+    double r[U], o[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long iq = i + q * T < n ? i + q * T : n - 1;
+      r[q] = rho[iq];
+      o[q] = PASS == 0 ? dr[iq] : ocp[iq];
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      if (i + q * T >= n) break;
+      if constexpr (PASS == 0) {
+        o[q] = oc_raw(r[q], o[q], A);
+        any = any || o[q] != 0.0;
+        o[q] = fmax(1e-12, o[q]);
+        ocp[i + q * T] = o[q];
+      }
+      oc_eval(r[q], allz ? 1e-3 : o[q], move, A, silam, v);
+    }
+  }
+  v[15] = any ? 1.0 : 0.0;
+  block_sum16(v, sw, ssum);
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    part[threadIdx.x * OC_MAX_BLOCKS + blockIdx.x] = ssum[threadIdx.x];
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!am_last) return;
+  __threadfence();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;  // 16 warps, one per value
+  double s = 0.0;
+  for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(part + wid * OC_MAX_BLOCKS + b);
+  s = warp_sum(s);
+  if (lane == 0) ssum[wid] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const unsigned ok = __ballot_sync(0xffffffffu, lane < OC_CAND && oc_feasible(ssum[lane & 15], vol, vf));
+    if (lane == 0) {
+      *ticket = 0u;
+      OcBis B = oc_start();
+      bool done = false;
+      if constexpr (PASS == 0) {
+        const bool some = ssum[15] != 0.0;  // no sensitivities: the passes that follow evaluate the fallback
+        st->allzero = some ? 0 : 1;
+        if (some) done = oc_move(B, true, ok, slam);
+      } else {
+        B = OcBis{st->l1, st->l2, st->last, st->a, st->b, st->steps};
+        done = oc_move(B, st->spread != 0, ok, slam);
+      }
+      st->l1 = B.l1;
+      st->l2 = B.l2;
+      st->last = B.last;
+      st->a = B.a;
+      st->b = B.b;
+      st->steps = B.steps;
+      st->done = done ? 1 : 0;
+      st->spread = oc_wide(B) ? 1 : 0;
+      sB = B;
+    }
+    __syncwarp();
+    if (lane < OC_CAND) st->lam[lane] = oc_candidate(sB, lane);
+  }
+}
+
+__global__ void __launch_bounds__(OC_THREADS)
+k_oc_design(long long n, const double* __restrict__ rho, const double* __restrict__ ocp, double move,
+            double* __restrict__ rho_new, double* part, unsigned* ticket, OcState* st, OcState* host) {
+  EDGE_PDL_ENTRY();
+  const double lam = st->last;
+  const bool allz = st->allzero != 0;
+  double acc = 0.0;
+  for (long long i = blockIdx.x * (long long)OC_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * OC_THREADS) {
+    const double r = rho[i];
+    const double x = oc_value(r, allz ? 1e-3 : ocp[i], lam, move);
+    rho_new[i] = x;
+    acc += (x - r) * (x - r);
+  }
+  __shared__ double sh[32];
+  const double bt = block_sum(acc, sh);
+  grid_reduce_finish(bt, part, ticket, [=](double t) {
+    st->change = t;
+    if (host) {
+      host->last = lam;
+      host->steps = st->steps;
+      host->change = t;
+    }
+  });
+}
+
+// The passes of k_oc_bisect by one thread block cluster of C blocks (C = 1: one block), for
+// element counts that leave most of the grid's passes waiting: the whole update is one launch,
+// a pass ends in a cluster barrier (the block sums go to every block's shared memory, which then
+// moves the bracket and forms the next candidates by itself) instead of a launch boundary.
+template <int C, int BT>
+EDGE_D void oc_team(const BatchOcDesc& d, double move, double& last, int& steps, double& change) {
+  constexpr int REG = 8;  // elements a thread keeps in registers
+  namespace cg = cooperative_groups;
+  __shared__ double sw[(BT / 32) * 16];
+  __shared__ double ssum[16], slam[16], silam[16];
+  __shared__ double sall[2][C][16];
+  __shared__ OcBis sB;
+  __shared__ int s_done, s_allz;
+  unsigned rank = 0;
+  if constexpr (C > 1) rank = cg::this_cluster().block_rank();
+  const long long i0 = rank * (long long)BT + threadIdx.x, T = (long long)C * BT;
+  int buf = 0;
+  // team sums of v[0..15] -> ssum (the same in every block)
+  auto team_sum = [&](double v[16]) {
+    block_sum16(v, sw, ssum);
+    __syncthreads();
+    if constexpr (C > 1) {
+      auto cl = cg::this_cluster();
+      for (int k = threadIdx.x; k < 16 * C; k += BT) *cl.map_shared_rank(&sall[buf][rank][k & 15], k >> 4) = ssum[k & 15];
+      cl.sync();
+      if (threadIdx.x < 16) {
+        double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < C; ++k) s4[k & 3] += sall[buf][k][threadIdx.x];
+        ssum[threadIdx.x] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      }
+      buf ^= 1;  // this buffer is written again two sums from now, behind the next sum's barrier
+      __syncthreads();
+    }
+  };
+  double rr[REG], oo[REG];
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < REG; ++q) {
+    const long long i = i0 + q * T;
+    rr[q] = oo[q] = 0.0;
+    if (i < d.n) {
+      rr[q] = d.rho[i];
+      const double o = oc_raw(rr[q], d.dr[i], d.A);
+      any = any || o != 0.0;
+      oo[q] = fmax(1e-12, o);
+    }
+  }
+  for (long long i = i0 + REG * T; i < d.n; i += T) {
+    const double o = oc_raw(d.rho[i], d.dr[i], d.A);
+    any = any || o != 0.0;
+    d.ocp[i] = fmax(1e-12, o);
+  }
+  if (threadIdx.x == 0) {
+    sB = oc_start();
+    s_done = 0;
+    s_allz = 0;
+  }
+  __syncthreads();
+  for (int pass = 0; pass < 200 && !s_done; ++pass) {
+    if (threadIdx.x < OC_CAND) {
+      const double lam = oc_candidate(sB, threadIdx.x);
+      slam[threadIdx.x] = lam;
+      silam[threadIdx.x] = 1.0 / lam;
+    }
+    __syncthreads();
+    const bool allz = s_allz != 0;
+    double v[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) v[t] = 0.0;
+#pragma unroll
+    for (int q = 0; q < REG; ++q)
+      if (i0 + q * T < d.n) oc_eval(rr[q], allz ? 1e-3 : oo[q], move, d.A, silam, v);
+    for (long long i = i0 + REG * T; i < d.n; i += T) oc_eval(d.rho[i], allz ? 1e-3 : d.ocp[i], move, d.A, silam, v);
+    v[15] = any ? 1.0 : 0.0;
+    team_sum(v);
+    if (threadIdx.x < 32) {
+      const unsigned ok = __ballot_sync(0xffffffffu, threadIdx.x < OC_CAND && oc_feasible(ssum[threadIdx.x & 15], d.vol, d.vf));
+      if (threadIdx.x == 0) {
+        OcBis B = sB;
+        if (pass == 0 && ssum[15] == 0.0)
+          s_allz = 1;  // no sensitivities: the passes that follow evaluate the fallback
+        else
+          s_done = oc_move(B, oc_wide(B), ok, slam) ? 1 : 0;
+        sB = B;
+      }
+    }
+    __syncthreads();
+  }
+  last = sB.last;
+  steps = sB.steps;
+  const bool allz = s_allz != 0;
+  double v[16];
+#pragma unroll
+  for (int t = 0; t < 16; ++t) v[t] = 0.0;
+#pragma unroll
+  for (int q = 0; q < REG; ++q) {
+    const long long i = i0 + q * T;
+    if (i < d.n) {
+      const double x = oc_value(rr[q], allz ? 1e-3 : oo[q], last, move);
+      d.rho_new[i] = x;
+      v[0] += (x - rr[q]) * (x - rr[q]);
+    }
+  }
+  for (long long i = i0 + REG * T; i < d.n; i += T) {
+    const double r = d.rho[i], x = oc_value(r, allz ? 1e-3 : d.ocp[i], last, move);
+    d.rho_new[i] = x;
+    v[0] += (x - r) * (x - r);
+  }
+  team_sum(v);  // every block has read its shared memory's remote writes when this returns
+  change = ssum[0];
+  __syncthreads();
+}
+
+constexpr int OC_TEAM = 16, OC_TEAM_THREADS = 512;
+__global__ void __launch_bounds__(OC_TEAM_THREADS)
+k_oc_cluster(BatchOcDesc d, double move, OcState* st, OcState* host) {
+  EDGE_PDL_ENTRY();
+  double last, change;
+  int steps;
+  oc_team<OC_TEAM, OC_TEAM_THREADS>(d, move, last, steps, change);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->last = last;
+    st->steps = steps;
+    st->change = change;
+    if (host) {
+      host->last = last;
+      host->steps = steps;
+      host->change = change;
+    }
+  }
+}
+
+// One block per problem, taken from a queue.
+constexpr int OCB_THREADS = 512;
+__global__ void __launch_bounds__(OCB_THREADS)
+k_oc_batch(const BatchOcDesc* D, int nprob, unsigned* queue, double move, double* lam_out, int* steps_out) {
+  __shared__ int s_idx;
+  for (;;) {
+    if (threadIdx.x == 0) s_idx = (int)atomicAdd(queue, 1u);
+    __syncthreads();
+    const int idx = s_idx;
+    __syncthreads();
+    if (idx >= nprob) return;
+    double last, change;
+    int steps;
+    oc_team<1, OCB_THREADS>(D[idx], move, last, steps, change);
+    if (threadIdx.x == 0) {
+      lam_out[idx] = last;
+      steps_out[idx] = steps;
+    }
+    __syncthreads();
+  }
+}
+
+// One cluster up to OC_CLUSTER_MAX elements, the whole grid beyond.  A call (with its host read) in
+// us, cluster / grid: 4,800 elements 54 / 73, 49,152 67 / 74, 65,536 73 / 68, 110,592 97 / 68,
+// 221,184 144 / 74: the cluster's 16 SMs run out of FP64 rate (four operations per element and
+// candidate), the grid's passes cost their launches whatever the size.  The launches with host
+// reads and divisions that both replace took 356 us at 4,800, 363 at 65,536, 776 at 524,288
+// (now 96) and 2,086 at 4.2M elements (now 309).
+constexpr long long OC_CLUSTER_MAX = 49152;
+
+int oc_launch(long long n, const double* rho, const double* dr, double A, double vol, double vf, double move,
+              double* ocp, double* rho_new, double* part, unsigned* ticket, OcState* st, OcState* host,
+              cudaStream_t stream) {
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = stream;
+  cfg.attrs = at;
+  if (n <= OC_CLUSTER_MAX) {
+    static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
+    if (!attr.load()) {
+      if (cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
+      attr = true;
+    }
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = OC_TEAM;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(OC_TEAM);
+    cfg.blockDim = dim3(OC_TEAM_THREADS);
+    cudaLaunchKernelEx(&cfg, k_oc_cluster, BatchOcDesc{n, rho, dr, ocp, rho_new, A, vol, vf}, move, st, host);
+    return 1;
+  }
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)std::min<long long>((n + OC_THREADS - 1) / OC_THREADS, OC_MAX_BLOCKS));
+  cfg.blockDim = dim3(OC_THREADS);
+  cfg.numAttrs = 0;  // the first pass follows whatever produced its inputs
+  cudaLaunchKernelEx(&cfg, k_oc_bisect<0>, n, rho, dr, A, vol, vf, move, ocp, part, ticket, st);
+  cfg.numAttrs = 1;
+  for (int p = 1; p < OC_PASSES; ++p)
+    cudaLaunchKernelEx(&cfg, p == 1 ? k_oc_bisect<1> : k_oc_bisect<2>, n, rho, dr, A, vol, vf, move, ocp, part, ticket, st);
+  cudaLaunchKernelEx(&cfg, k_oc_design, n, rho, (const double*)ocp, move, rho_new, part, ticket, st, host);
+  return OC_PASSES + 1;
+}
+
+int oc_batch_launch(const BatchOcDesc* D, int nprob, unsigned* queue, double move, double* lam_out, int* steps_out,
+                    cudaStream_t stream) {
+  k_oc_batch<<<std::max(1, std::min(nprob, 148)), OCB_THREADS, 0, stream>>>(D, nprob, queue, move, lam_out, steps_out);
+  return 1;
+}
+
+}  // namespace edge

@@ -837,158 +837,12 @@ __global__ void k_dk2(const Geo g, const double* __restrict__ U, const double* _
   dk[e] = val;
 }
 
-// ------------------------------------------------------------------ OC bisection (TopOpt/_cuda.py:242-280)
-// ocP = max(1e-12, rho * sqrt(max(-dr/A, 0))) with NaN -> 0; the all-zero fallback of
-// MaterialModels.py:87-88 is applied by k_oc_fallback when sum(ocP_raw) == 0.
-__global__ void k_oc_prep(long long n, const double* __restrict__ rho, const double* __restrict__ dr, double A,
-                          double* __restrict__ ocp, double* part, unsigned* ticket, double* sum_dst) {
-  EDGE_PDL_ENTRY();
-  double acc = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double v = rho[i] * sqrt(fmax(-dr[i] / A, 0.0));
-    if (isnan(v)) v = 0.0;
-    acc += fabs(v);
-    ocp[i] = v;
-  }
-  __shared__ double sh[32];
-  double bt = block_sum(acc, sh);
-  grid_reduce_finish(bt, part, ticket, DotSink{sum_dst});
-}
-
-__global__ void k_oc_floor(long long n, double* __restrict__ ocp, const double* __restrict__ sum) {
-  EDGE_PDL_ENTRY();
-  const bool allzero = (*sum == 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double v = allzero ? 1e-3 : ocp[i];
-    ocp[i] = fmax(1e-12, v);
-  }
-}
-
-constexpr int OC_DEPTH = 4;                  // bisection levels resolved per pass
-constexpr int OC_NODES = (1 << OC_DEPTH) - 1;
-struct OcState {
-  double l1, l2, last;
-  double vf, vol;
-  int steps, done;
-  double sums[OC_NODES];
-};
-
+// ------------------------------------------------------------------ OC value (TopOpt/_cuda.py:262-267)
+// The design value at multiplier lam: o / lam within the move limits and [0, 1].
 EDGE_D double oc_rho(double r, double o, double lam, double move) {
   const double xU = fmin(fmax(r + move, 0.0), 1.0);
   const double xL = fmin(fmax(r - move, 0.0), 1.0);
   return fmax(0.0, fmax(xL, fmin(1.0, fmin(xU, o / lam))));
-}
-
-// Evaluate sum(rho_new(lambda) * A) at every node of the next OC_DEPTH levels of the
-// bisection tree.  Tree node t (heap order): children 2t+1 (volume ok -> l2 = mid)
-// and 2t+2 (l1 = mid).
-__global__ void __launch_bounds__(256) k_oc_pass(long long n, const double* __restrict__ rho, const double* __restrict__ ocp,
-                                                 double A, double move, OcState* st, double* part, unsigned* ticket) {
-  EDGE_PDL_ENTRY();
-  if (st->done) return;
-  double lam[OC_NODES];
-  {
-    double L1[OC_NODES], L2[OC_NODES];
-    L1[0] = st->l1;
-    L2[0] = st->l2;
-    for (int t = 0; t < OC_NODES; ++t) {
-      lam[t] = 0.5 * (L1[t] + L2[t]);
-      if (2 * t + 2 < OC_NODES) {
-        L1[2 * t + 1] = L1[t];
-        L2[2 * t + 1] = lam[t];
-        L1[2 * t + 2] = lam[t];
-        L2[2 * t + 2] = L2[t];
-      }
-    }
-  }
-  double acc[OC_NODES];
-  for (int t = 0; t < OC_NODES; ++t) acc[t] = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double r = rho[i], o = ocp[i];
-    for (int t = 0; t < OC_NODES; ++t) acc[t] += oc_rho(r, o, lam[t], move) * A;
-  }
-  __shared__ double sh[32];
-  __shared__ double bsum[OC_NODES];
-  for (int t = 0; t < OC_NODES; ++t) {
-    double v = block_sum(acc[t], sh);
-    if (threadIdx.x == 0) bsum[t] = v;
-  }
-  __syncthreads();
-  // grid-wide: partials laid out [block][t]
-  __shared__ bool am_last;
-  const unsigned nblk = gridDim.x;
-  if (threadIdx.x == 0) {
-    for (int t = 0; t < OC_NODES; ++t) part[(long long)blockIdx.x * OC_NODES + t] = bsum[t];
-    __threadfence();
-    am_last = (atomicAdd(ticket, 1u) == nblk - 1);
-  }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  for (int t = 0; t < OC_NODES; ++t) {
-    double a = 0.0;
-    for (unsigned b = threadIdx.x; b < nblk; b += blockDim.x) a += ((volatile double*)part)[(long long)b * OC_NODES + t];
-    double tot = block_sum(a, sh);
-    if (threadIdx.x == 0) st->sums[t] = tot;
-  }
-  if (threadIdx.x == 0) {
-    // walk the tree exactly as the sequential bisection would
-    int t = 0;
-    double l1 = st->l1, l2 = st->l2;
-    for (int d = 0; d < OC_DEPTH; ++d) {
-      if (!((l2 - l1) / (l2 + l1) > 1e-4)) {
-        st->done = 1;
-        break;
-      }
-      const double mid = 0.5 * (l1 + l2);
-      const bool valid = (st->sums[t] / st->vol <= st->vf);
-      if (valid) l2 = mid;
-      else l1 = mid;
-      st->last = mid;
-      st->steps += 1;
-      t = 2 * t + (valid ? 1 : 2);
-    }
-    st->l1 = l1;
-    st->l2 = l2;
-    if (!((l2 - l1) / (l2 + l1) > 1e-4)) st->done = 1;
-    *ticket = 0u;
-  }
-}
-
-// rho_new at the last lambda tried; also sum((rho_new - rho)^2) for the RMS change.
-__global__ void k_oc_final(long long n, const double* __restrict__ rho, const double* __restrict__ ocp, double move,
-                           const OcState* st, double* __restrict__ rho_new, double* part, unsigned* ticket,
-                           double* chg_dst) {
-  EDGE_PDL_ENTRY();
-  const double lam = st->last;
-  double acc = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double r = rho[i];
-    const double v = oc_rho(r, ocp[i], lam, move);
-    rho_new[i] = v;
-    acc += (v - r) * (v - r);
-  }
-  __shared__ double sh[32];
-  double bt = block_sum(acc, sh);
-  grid_reduce_finish(bt, part, ticket, DotSink{chg_dst});
-}
-
-// Start state of one OC bisection on the device: bracket [1e-9, 1e9] (TopOpt/_cuda.py:260-261).
-__global__ void k_oc_state_init(OcState* st, double vf, double vol) {
-  EDGE_PDL_ENTRY();
-  OcState init{};
-  init.l1 = 1e-9;
-  init.l2 = 1e9;
-  init.last = 0.5 * (init.l1 + init.l2);
-  init.vf = vf;
-  init.vol = vol;
-  *st = init;
-}
-// Condition of the OC loop inside a graph: bisect again while the bracket is open and fewer
-// than max_steps bisection steps ran (the bound of the host loop).
-__global__ void k_cond_oc(cudaGraphConditionalHandle h, const OcState* st, int max_steps) {
-  EDGE_PDL_ENTRY();
-  cudaGraphSetConditional(h, (st->done == 0 && st->steps < max_steps) ? 1u : 0u);
 }
 
 // Multi-material SIMP law (PenalizedMultiMaterial, MaterialModels.py:102-205).  rho is the

@@ -24,6 +24,7 @@
 #include "coarse.cuh"
 #include "common.cuh"
 #include "element_op.cuh"
+#include "fields.cuh"
 #include "fine_apply.cuh"
 #include "fine_tma.cuh"
 #include "fine_pk.cuh"
@@ -258,7 +259,7 @@ struct Prob {
   cudaGraph_t it_graph = nullptr;
   cudaGraphExec_t it_exec = nullptr;
   std::vector<double> it_key;
-  long long it_fixed = 0, it_oc_body = 0, it_body = 0, it_rep = 0;
+  long long it_fixed = 0, it_body = 0, it_rep = 0;
   double *it_rho = nullptr, *it_dr = nullptr, *it_rho_new = nullptr, *it_dr_new = nullptr;
   std::vector<double> sg_key;
   long long sg_pro = 0, sg_body = 0, sg_if = 0;  // launches per section, for the launch tally
@@ -2020,12 +2021,10 @@ struct edge_filter {
 };
 
 // One SIMP iteration as one CUDA graph: the OC update of (it_rho, it_dr) into it_rho_new
-// (prep, floor, bracket init, the bisection passes as a while node whose condition a kernel
-// sets from the device-side state, the final design), then the analysis of it_rho_new:
+// (oc_launch: a fixed sequence of passes), then the analysis of it_rho_new:
 // filter + SIMP law, the solve (hierarchy set-up and PCG loop as in capture_solve),
 // compliance, sensitivities and the filter transpose into it_dr_new.  Every buffer is the
 // problem's own; the caller copies the user's arrays in and out around the launch.
-static const int OC_MAX_STEPS = 200;  // the host loop's bound (edge_oc_update)
 static void capture_iteration(Prob& P, const edge_filter& F, double A, double vol, double vf, double move,
                               double penalty, double void_, double tol, int maxiter) {
   if (P.it_exec) {
@@ -2038,58 +2037,21 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
   }
   const Geo& g = P.g0;
   const long long n = P.n_el;
-  const unsigned nb = std::min<unsigned>(ew_blocks(n), 1024);
-  const unsigned nbp = std::min<unsigned>(nb, (unsigned)(P.part_cap / OC_NODES));
   const unsigned nbe = cdiv(P.n_el, 256);
   const long long nv = (long long)g.dof * g.n;
-  long long n_fixed0 = 0, n_fixed1 = 0, n_fixed2 = 0, n_ocb = 0;
+  long long n_fixed0 = 0, n_fixed1 = 0;
   SolveCounts sc;
   P.it_graph = capture_graph(P, [&](int& depth) {
     const long long a0 = P.nlaunch;
-    {
-      CatScope cat(P, CAT_OC);
-      launch(P, k_oc_prep, nb, 256, 0, n, (const double*)P.it_rho, (const double*)P.it_dr, A, P.ocp, P.part,
-             P.ticket, P.scal);
-      launch(P, k_oc_floor, nb, 256, 0, n, P.ocp, (const double*)P.scal);
-      launch(P, k_oc_state_init, 1, 1, 0, P.oc, vf, vol);
-      cudaStreamCaptureStatus cs;
-      cudaGraph_t gg;
-      const cudaGraphNode_t* deps;
-      size_t nd;
-      CK(cudaStreamGetCaptureInfo(P.cap[0], &cs, nullptr, &gg, &deps, &nd));
-      cudaGraphConditionalHandle ho;
-      CK(cudaGraphConditionalHandleCreate(&ho, gg, 0, cudaGraphCondAssignDefault));
-      launch(P, k_cond_oc, 1, 1, 0, ho, (const OcState*)P.oc, OC_MAX_STEPS);
-      CK(cudaStreamGetCaptureInfo(P.cap[0], &cs, nullptr, &gg, &deps, &nd));
-      cudaGraphNodeParams wp = {};
-      wp.type = cudaGraphNodeTypeConditional;
-      wp.conditional.handle = ho;
-      wp.conditional.type = cudaGraphCondTypeWhile;
-      wp.conditional.size = 1;
-      cudaGraphNode_t wnode;
-      CK(cudaGraphAddNode(&wnode, gg, deps, nd, &wp));
-      CK(cudaStreamUpdateCaptureDependencies(P.cap[0], &wnode, 1, cudaStreamSetCaptureDependencies));
-      P.stream = P.cap[1];
-      CK(cudaStreamBeginCaptureToGraph(P.cap[1], wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                       cudaStreamCaptureModeThreadLocal));
-      depth = 2;
-      const long long b0 = P.nlaunch;
-      launch(P, k_oc_pass, nbp, 256, 0, n, (const double*)P.it_rho, (const double*)P.ocp, A, move, P.oc, P.part,
-             P.ticket);
-      launch(P, k_cond_oc, 1, 1, 0, ho, (const OcState*)P.oc, OC_MAX_STEPS);
-      n_ocb = P.nlaunch - b0;
-      CK(cudaStreamEndCapture(P.cap[1], nullptr));
-      depth = 1;
-      P.stream = P.cap[0];
-      launch(P, k_oc_final, nb, 256, 0, n, (const double*)P.it_rho, (const double*)P.ocp, move, (const OcState*)P.oc,
-             P.it_rho_new, P.part, P.ticket, P.scal + 1);
-    }
+    P.nlaunch += oc_launch(n, P.it_rho, P.it_dr, A, vol, vf, move, P.ocp, P.it_rho_new, P.part, P.ticket, P.oc,
+                           nullptr, P.stream);
+    KCHECK();
     {
       CatScope cat(P, CAT_SENS);
       launch(P, k_filter_material<double, float>, nbe, 256, 0, g, F.taps, (const double*)P.it_rho_new, P.rho_f,
              P.E64, P.E32, penalty, void_, 0);
     }
-    n_fixed0 = P.nlaunch - a0 - n_ocb;
+    n_fixed0 = P.nlaunch - a0;
     sc = capture_solve_into(P, tol, maxiter, false, depth);
     const long long c0 = P.nlaunch;
     {
@@ -2103,9 +2065,7 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
     n_fixed1 = P.nlaunch - c0;
   });
   CK(cudaGraphInstantiate(&P.it_exec, P.it_graph, 0));
-  (void)n_fixed2;
   P.it_fixed = n_fixed0 + n_fixed1 + sc.pro;
-  P.it_oc_body = n_ocb;
   P.it_body = sc.body;
   P.it_rep = sc.rep;
 }
@@ -2166,12 +2126,10 @@ static void gen_matvec(edge_gen& M, const double* u, double* out, double* dot) {
 // file-scope device array, so the call allocates nothing.  One workspace per device: calls
 // whose work overlaps on one device (two streams, two host threads) race on it.
 constexpr long long OC_STATIC_MAX_EL = 1LL << 20;   // elements; the ocP cache is 8 MiB
-constexpr unsigned OC_STATIC_MAX_BLOCKS = 1024;     // reduction partials, as edge_oc_update
 struct OcStaticScratch {
-  OcState st;                                  // bisection state, rewritten by k_oc_static_init
-  double scal[2];                              // sum(ocP_raw), sum((rho_new - rho)^2)
-  unsigned ticket;                             // grid-reduction counter: zero when a kernel starts
-  double part[OC_STATIC_MAX_BLOCKS * OC_NODES];
+  OcState st;                                  // bisection state, rewritten by every call
+  unsigned ticket;                             // reduction counter: zero when a kernel starts
+  double part[OC_PART];
   double ocp[OC_STATIC_MAX_EL];
 };
 static __device__ __align__(256) OcStaticScratch g_oc_scratch;
@@ -2195,21 +2153,6 @@ static OcStaticScratch* oc_static_scratch(cudaStream_t stream) {
   if (e != cudaSuccess || !ptr)
     fail(EDGE_ECUDA, std::string("cudaGetSymbolAddress(OC workspace): ") + cudaGetErrorString(e));
   return static_cast<OcStaticScratch*>(ptr);
-}
-
-// Start state of one OC update: bracket [1e-9, 1e9] (TopOpt/_cuda.py:260-261), counter zero.
-__global__ void k_oc_static_init(OcStaticScratch* s, double vf, double vol) {
-  EDGE_PDL_ENTRY();
-  OcState init{};
-  init.l1 = 1e-9;
-  init.l2 = 1e9;
-  init.last = 0.5 * (init.l1 + init.l2);
-  init.vf = vf;
-  init.vol = vol;
-  s->st = init;
-  s->scal[0] = 0.0;
-  s->scal[1] = 0.0;
-  s->ticket = 0u;
 }
 
 #define API_BEGIN try {
@@ -3288,37 +3231,12 @@ static void oc_run(Prob& P, long long n, const double* rho, const double* dr, do
                    double move, double* rho_new) {
   CatScope cat(P, CAT_OC);
   if (n != P.n_el) fail(EDGE_EINVAL, "OC vector length does not match the number of elements");
-  const unsigned nb = std::min<unsigned>(ew_blocks(n), 1024);
-  launch(P, k_oc_prep, nb, 256, 0, n, rho, dr, A, P.ocp, P.part, P.ticket, P.scal);
-  launch(P, k_oc_floor, nb, 256, 0, n, P.ocp, P.scal);
-  OcState init{};
-  init.l1 = 1e-9;
-  init.l2 = 1e9;
-  init.last = 0.5 * (init.l1 + init.l2);
-  init.vf = vf;
-  init.vol = vol;
-  *P.oc_h = init;
-  CK(cudaMemcpyAsync(P.oc, P.oc_h, sizeof(OcState), cudaMemcpyHostToDevice, P.stream));
-  const unsigned nbp = std::min<unsigned>(nb, (unsigned)(P.part_cap / OC_NODES));
-  const int max_pass = (200 + OC_DEPTH - 1) / OC_DEPTH;
-  for (int pass = 0; pass < max_pass; ++pass) {
-    launch(P, k_oc_pass, nbp, 256, 0, n, rho, P.ocp, A, move, P.oc, P.part, P.ticket);
-    if ((pass & 3) == 3) {
-      CK(cudaMemcpyAsync(P.oc_h, P.oc, sizeof(OcState), cudaMemcpyDeviceToHost, P.stream));
-      CK(cudaStreamSynchronize(P.stream));
-      if (P.oc_h->done) break;
-    }
-  }
+  P.nlaunch += oc_launch(n, rho, dr, A, vol, vf, move, P.ocp, rho_new, P.part, P.ticket, P.oc, P.oc_h, P.stream);
   KCHECK();
-  launch(P, k_oc_final, nb, 256, 0, n, rho, P.ocp, move, P.oc, rho_new, P.part, P.ticket, P.scal + 1);
-  KCHECK();
-  CK(cudaMemcpyAsync(P.oc_h, P.oc, sizeof(OcState), cudaMemcpyDeviceToHost, P.stream));
-  CK(cudaMemcpyAsync(P.scal_h, P.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, P.stream));
   CK(cudaStreamSynchronize(P.stream));
 }
 
 
-// ---- unstructured meshes (kernels/_cuda.py:305-815, solvers/_gpu.py:11-58, geom/_filters.py:278-298)
 int edge_gen_create(int dof, long long n_nodes, long long n_el, const int* elem_ptr, const int* elem_flat,
                     const double* K, const long long* K_ptr, edge_gen** out) {
   API_BEGIN
@@ -3549,7 +3467,7 @@ int edge_oc_update(edge_problem* p, const double* rho_dev, const double* dr_dev,
   oc_run(P, P.n_el, rho_dev, dr_dev, A, vol, vf, move, rho_new_dev);
   if (lambda_out) *lambda_out = P.oc_h->last;
   if (steps_out) *steps_out = P.oc_h->steps;
-  if (sqchange_out) *sqchange_out = P.scal_h[1];
+  if (sqchange_out) *sqchange_out = P.oc_h->change;
   API_END
 }
 
@@ -3564,31 +3482,15 @@ int edge_oc_update_static(long long n, const double* rho_dev, const double* dr_d
                           std::to_string(OC_STATIC_MAX_EL) + " elements); use edge_oc_update");
   cudaStream_t st = (cudaStream_t)stream;
   OcStaticScratch* s = oc_static_scratch(st);
-  const unsigned nb = std::min<unsigned>(ew_blocks(n), OC_STATIC_MAX_BLOCKS);
-  k_oc_static_init<<<1, 1, 0, st>>>(s, vf, vol);
-  k_oc_prep<<<nb, 256, 0, st>>>(n, rho_dev, dr_dev, A, s->ocp, s->part, &s->ticket, &s->scal[0]);
-  k_oc_floor<<<nb, 256, 0, st>>>(n, s->ocp, &s->scal[0]);
+  CK(cudaMemsetAsync(&s->ticket, 0, sizeof(unsigned), st));
+  oc_launch(n, rho_dev, dr_dev, A, vol, vf, move, s->ocp, rho_new_dev, s->part, &s->ticket, &s->st, nullptr, st);
   KCHECK();
   OcState h{};
-  const int max_pass = (200 + OC_DEPTH - 1) / OC_DEPTH;
-  for (int pass = 0; pass < max_pass; ++pass) {
-    k_oc_pass<<<nb, 256, 0, st>>>(n, rho_dev, s->ocp, A, move, &s->st, s->part, &s->ticket);
-    if ((pass & 3) == 3) {
-      KCHECK();
-      CK(cudaMemcpyAsync(&h, &s->st, sizeof(OcState), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      if (h.done) break;
-    }
-  }
-  k_oc_final<<<nb, 256, 0, st>>>(n, rho_dev, s->ocp, move, &s->st, rho_new_dev, s->part, &s->ticket, &s->scal[1]);
-  KCHECK();
-  double chg = 0.0;
   CK(cudaMemcpyAsync(&h, &s->st, sizeof(OcState), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&chg, &s->scal[1], sizeof(double), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (lambda_out) *lambda_out = h.last;
   if (steps_out) *steps_out = h.steps;
-  if (sqchange_out) *sqchange_out = chg;
+  if (sqchange_out) *sqchange_out = h.change;
   API_END
 }
 
@@ -3646,9 +3548,7 @@ int edge_simp_iteration(edge_problem* p, edge_filter* f, const double* rho_dev, 
   check_err(P);
   P.last_iters = P.st_h->iter;
   P.last_true_res = (P.prec != EDGE_FP64) ? 1 + P.st_h->n_true : 0;
-  const long long passes = (P.oc_h->steps + OC_DEPTH - 1) / OC_DEPTH;
-  P.nlaunch += P.it_fixed + P.it_body * (long long)P.st_h->iter + P.it_rep * (long long)P.st_h->n_true +
-               P.it_oc_body * passes;
+  P.nlaunch += P.it_fixed + P.it_body * (long long)P.st_h->iter + P.it_rep * (long long)P.st_h->n_true;
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, P.ev[0], P.ev[2]));
   P.last_setup_ms = 0.0;
@@ -3658,7 +3558,7 @@ int edge_simp_iteration(edge_problem* p, edge_filter* f, const double* rho_dev, 
   if (iters_out) *iters_out = P.st_h->iter;
   if (lambda_out) *lambda_out = P.oc_h->last;
   if (oc_steps_out) *oc_steps_out = P.oc_h->steps;
-  if (sqchange_out) *sqchange_out = P.scal_h[1];
+  if (sqchange_out) *sqchange_out = P.oc_h->change;
   API_END
 }
 
@@ -3985,13 +3885,8 @@ int edge_batch_oc_update(edge_batch* b, const double* const* rho, const double* 
   try {
     CK(cudaMemcpyAsync(B.d_oc, B.h_oc, n * sizeof(BatchOcDesc), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(B.queue, 0, sizeof(unsigned), s));
-    int per_sm = 0, sms = 0, dev = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_oc<512>, 512, 0));
-    const int grid = std::max(1, std::min(n, std::max(1, per_sm) * sms));
-    launch(P0, k_batch_oc<512>, dim3(grid), dim3(512), 0, (const BatchOcDesc*)B.d_oc, n, B.queue, move, B.d_res,
-           B.d_iters);
+    P0.nlaunch += oc_batch_launch(B.d_oc, n, B.queue, move, B.d_res, B.d_iters, s);
+    KCHECK();
   } catch (...) {
     P0.stream = saved0;
     throw;

@@ -292,7 +292,7 @@ class CuTopOpt:
         ``solve_and_process(rho_new, iteration)``, returning (rho_new, compliance, dr, residual).
         With this package's objects (and once the solver's autotuners have run, on the first
         analyses) the two run as one CUDA graph launch with one host read
-        (edge_simp_iteration: the OC bisection loop is a device-side conditional node);
+        (edge_simp_iteration: the OC update is a fixed sequence of launches);
         otherwise as the two calls."""
         sv = self.solver
         ready = (self.fused and self.n_sets == 1 and self.reuse_sol and sv.graph and sv.last_x0 is not None

@@ -325,8 +325,8 @@ int edge_simp_solve_and_process(edge_problem* p, edge_filter* f, const double* r
 
 /* ---- one whole SIMP iteration as one CUDA graph launch.  Replaces TopOpt.update_design
  * followed by TopOpt.solve_and_process (TopOpt/_cuda.py:242-302) for SingleMaterial: the OC
- * update of rho_dev with the sensitivities dr_dev (the bisection loop runs on the device as a
- * conditional node: no host read inside it) into rho_new_dev, then the analysis of rho_new_dev
+ * update of rho_dev with the sensitivities dr_dev (a fixed sequence of launches, no host read
+ * between them) into rho_new_dev, then the analysis of rho_new_dev
  * exactly as edge_simp_solve_and_process (new sensitivities into dr_new_dev, U_dev updated,
  * the filtered density into rho_f_dev when given).  The host reads the results once.  The
  * graph is captured on the first call and again when a setting baked into it changes; the
