@@ -44,8 +44,8 @@ def _stale():
 
 
 def build(force=False, verbose=False, extra=()):
-    """Compile every stale source to an object (in parallel, each with parallel code
-    generation) and link the library."""
+    """Compile every stale source to an object (in parallel)
+    and link the library."""
     if not force and not _stale():
         return LIB
     os.makedirs(OBJDIR, exist_ok=True)
@@ -56,7 +56,7 @@ def build(force=False, verbose=False, extra=()):
         path, obj = os.path.join(CSRC, src), os.path.join(OBJDIR, src + ".o")
         objs.append(obj)
         if force or extra or _older(obj, [path] + _headers()):
-            cmd = [nvcc_path(), "-c", *flags, "--split-compile", "0", *extra, "-o", obj + ".tmp", path]
+            cmd = [nvcc_path(), "-c", *flags, *extra, "-o", obj + ".tmp", path]
             if verbose:
                 print(" ".join(cmd), flush=True)
             jobs.append((obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))

@@ -38,4 +38,42 @@ struct BatchOcDesc {
 int oc_batch_launch(const BatchOcDesc* D, int nprob, unsigned* queue, double move, double* lam_out, int* steps_out,
                     cudaStream_t stream);
 
+// ------------------------------------------------------------------ density filter
+// Cone filter (geom/_filters.py:72-161, core/_filter.py:78-124): taps o_k with global weights w_k;
+// (H rho)_e = sum_k w_k rho_{e+o_k} / N_e with N_e = sum of the in-bounds w_k.
+constexpr int MAX_TAPS = 128;
+struct Taps {
+  int n;
+  int off[MAX_TAPS][3];  // (dx, dy, dz) in element units
+  double w[MAX_TAPS];
+};
+// The taps by columns along the middle element axis (y in 3-D, x in 2-D) for the tiled kernels:
+// column c is at offset (o0, o2) of the slowest and fastest axis and holds the weights of the
+// middle offsets -R..R (present: bit b for offset b - R).
+constexpr int FT_RMAX = 3;
+constexpr int FT_COLS = (2 * FT_RMAX + 1) * (2 * FT_RMAX + 1);
+struct TapCols {
+  int n, R, R0;  // columns; tile halo along the middle and fastest axes, along the slowest
+  double nint;   // N_e of an element whose taps are all in bounds
+  signed char o0[FT_COLS], o2[FT_COLS];
+  unsigned char present[FT_COLS];
+  double w[FT_COLS][2 * FT_RMAX + 1];
+};
+// false when a tap repeats or reaches further than FT_RMAX: the one-thread-per-element kernels
+bool make_tap_cols(int dim, const Taps& t, TapCols& c);
+// What the forward filter stores: H rho, and for the SIMP law (MaterialModels.py:47-60) the
+// penalised density clip((H rho)^p, void, 1) at the element's slot of `slots`.
+struct FilterOut {
+  double* rho_f;
+  double* E64;  // null: no law
+  float* E32;   // may be null
+  double penalty, vmin;
+  Geo slots;    // node grid of the element slots (rows may be longer than the filter's grid)
+};
+int filter_forward(const Geo& g, const Taps& t, const TapCols* c, const double* N, const double* in,
+                   const FilterOut& out, cudaStream_t stream);
+int filter_transpose(const Geo& g, const Taps& t, const TapCols* c, const double* N, const double* in, double* out,
+                     cudaStream_t stream);
+int filter_norm(const Geo& g, const Taps& t, double* N, cudaStream_t stream);
+
 }  // namespace edge

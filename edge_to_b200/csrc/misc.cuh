@@ -148,140 +148,6 @@ __global__ void k_elem_user_to_slots_emb(const Geo g, const Geo gr, const double
   v[s] = Conv<TO>::from(val);
 }
 
-// ------------------------------------------------------------------ density filter
-// Cone filter (geom/_filters.py:72-161, core/_filter.py:78-124): taps o_k with global
-// weights w_k; (H rho)_e = sum_k w_k rho_{e+o_k} / sum_{in-bounds k} w_k.
-constexpr int MAX_TAPS = 128;
-struct Taps {
-  int n;
-  int off[MAX_TAPS][3];  // (dx, dy, dz) in element units
-  double w[MAX_TAPS];
-};
-
-// Forward filter fused with the SIMP law (MaterialModels.py:47-60):
-//   rho_f = H rho (user order), E = clip(rho_f^p, void, 1) written in slot layout
-//   (types TE1 and optional TE2 for a second precision).
-template <typename TE1, typename TE2>
-__global__ void k_filter_material(const Geo g, const Taps taps, const double* __restrict__ rho,
-                                  double* __restrict__ rho_f, TE1* __restrict__ E1, TE2* __restrict__ E2,
-                                  double penalty, double vmin, int plain) {
-  EDGE_PDL_ENTRY();
-  const int nelx = g.nx - 1, nely = g.ny - 1, nelz = g.dim == 3 ? g.nz - 1 : 1;
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nel = (long long)nelx * nely * nelz;
-  if (e >= nel) return;
-  int i, j, k;
-  if (g.dim == 3) {
-    k = (int)(e % nelz);
-    j = (int)((e / nelz) % nely);
-    i = (int)(e / ((long long)nelz * nely));
-  } else {
-    k = 0;
-    j = (int)(e % nely);
-    i = (int)(e / nely);
-  }
-  double sv = 0.0, sw = 0.0;
-  for (int t = 0; t < taps.n; ++t) {
-    const int ii = i + taps.off[t][0], jj = j + taps.off[t][1], kk = k + taps.off[t][2];
-    if (ii < 0 || ii >= nelx || jj < 0 || jj >= nely || kk < 0 || kk >= nelz) continue;
-    const double w = taps.w[t];
-    sv += w * __ldg(rho + user_elem(g, ii, jj, kk));
-    sw += w;
-  }
-  const double rf = sw > 0.0 ? sv / sw : 0.0;
-  rho_f[e] = rf;
-  double Ev;
-  if (plain) {
-    Ev = fmin(fmax(rf, vmin), 1.0);
-  } else {
-    Ev = fmin(fmax(pow(rf, penalty), vmin), 1.0);
-  }
-  const long long s = g.dim == 3 ? g.slot3(i, j, k) : g.slot2(i, j);
-  E1[s] = Conv<TE1>::from(Ev);
-  if (E2) E2[s] = Conv<TE2>::from(Ev);
-}
-
-// Filter only (H rho), user order in and out.
-__global__ void k_filter(const Geo g, const Taps taps, const double* __restrict__ in, double* __restrict__ out) {
-  EDGE_PDL_ENTRY();
-  const int nelx = g.nx - 1, nely = g.ny - 1, nelz = g.dim == 3 ? g.nz - 1 : 1;
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nel = (long long)nelx * nely * nelz;
-  if (e >= nel) return;
-  int i, j, k;
-  if (g.dim == 3) {
-    k = (int)(e % nelz);
-    j = (int)((e / nelz) % nely);
-    i = (int)(e / ((long long)nelz * nely));
-  } else {
-    k = 0;
-    j = (int)(e % nely);
-    i = (int)(e / nely);
-  }
-  double sv = 0.0, sw = 0.0;
-  for (int t = 0; t < taps.n; ++t) {
-    const int ii = i + taps.off[t][0], jj = j + taps.off[t][1], kk = k + taps.off[t][2];
-    if (ii < 0 || ii >= nelx || jj < 0 || jj >= nely || kk < 0 || kk >= nelz) continue;
-    sv += taps.w[t] * __ldg(in + user_elem(g, ii, jj, kk));
-    sw += taps.w[t];
-  }
-  out[e] = sw > 0.0 ? sv / sw : 0.0;
-}
-
-// Normaliser N_e = sum of in-bounds weights (core/_filter.py:6-40).
-__global__ void k_filter_norm(const Geo g, const Taps taps, double* __restrict__ N) {
-  EDGE_PDL_ENTRY();
-  const int nelx = g.nx - 1, nely = g.ny - 1, nelz = g.dim == 3 ? g.nz - 1 : 1;
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nel = (long long)nelx * nely * nelz;
-  if (e >= nel) return;
-  int i, j, k;
-  if (g.dim == 3) {
-    k = (int)(e % nelz);
-    j = (int)((e / nelz) % nely);
-    i = (int)(e / ((long long)nelz * nely));
-  } else {
-    k = 0;
-    j = (int)(e % nely);
-    i = (int)(e / nely);
-  }
-  double sw = 0.0;
-  for (int t = 0; t < taps.n; ++t) {
-    const int ii = i + taps.off[t][0], jj = j + taps.off[t][1], kk = k + taps.off[t][2];
-    if (ii < 0 || ii >= nelx || jj < 0 || jj >= nely || kk < 0 || kk >= nelz) continue;
-    sw += taps.w[t];
-  }
-  N[e] = sw;
-}
-
-// Transpose: (H^T v)_e = sum_k (w_k / N_{e+o_k}) v_{e+o_k} (core/_filter.py:42-76).
-__global__ void k_filter_T(const Geo g, const Taps taps, const double* __restrict__ N, const double* __restrict__ in,
-                           double* __restrict__ out) {
-  EDGE_PDL_ENTRY();
-  const int nelx = g.nx - 1, nely = g.ny - 1, nelz = g.dim == 3 ? g.nz - 1 : 1;
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nel = (long long)nelx * nely * nelz;
-  if (e >= nel) return;
-  int i, j, k;
-  if (g.dim == 3) {
-    k = (int)(e % nelz);
-    j = (int)((e / nelz) % nely);
-    i = (int)(e / ((long long)nelz * nely));
-  } else {
-    k = 0;
-    j = (int)(e % nely);
-    i = (int)(e / nely);
-  }
-  double sv = 0.0;
-  for (int t = 0; t < taps.n; ++t) {
-    const int ii = i + taps.off[t][0], jj = j + taps.off[t][1], kk = k + taps.off[t][2];
-    if (ii < 0 || ii >= nelx || jj < 0 || jj >= nely || kk < 0 || kk >= nelz) continue;
-    const long long q = user_elem(g, ii, jj, kk);
-    sv += (taps.w[t] / __ldg(N + q)) * __ldg(in + q);
-  }
-  out[e] = sv;
-}
-
 // ------------------------------------------------------------------ sensitivities
 // dk_e = -u_e^T K0 u_e (core/_ops.py:5-13) from the solution in slot layout, and
 // optionally g_e = p clip(rho_f, void, 1)^(p-1) dk_e (MaterialModels.py:62-73).

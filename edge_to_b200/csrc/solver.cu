@@ -2013,8 +2013,11 @@ struct edge_problem {
 struct edge_filter {
   Geo g;
   Taps taps;
+  TapCols cols;
+  bool tiled = false;  // cols describes the taps
   double* N = nullptr;
   long long n_el = 0;
+  const TapCols* tile() const { return tiled ? &cols : nullptr; }
   ~edge_filter() {
     if (N) cudaFree(N);
   }
@@ -2048,8 +2051,9 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
     KCHECK();
     {
       CatScope cat(P, CAT_SENS);
-      launch(P, k_filter_material<double, float>, nbe, 256, 0, g, F.taps, (const double*)P.it_rho_new, P.rho_f,
-             P.E64, P.E32, penalty, void_, 0);
+      P.nlaunch += filter_forward(F.g, F.taps, F.tile(), F.N, P.it_rho_new,
+                                  FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, g}, P.stream);
+      KCHECK();
     }
     n_fixed0 = P.nlaunch - a0;
     sc = capture_solve_into(P, tol, maxiter, false, depth);
@@ -2060,7 +2064,8 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
              (const double*)P.x64, P.part, P.ticket, P.scal + 2);
       launch(P, k_dk<double>, nbe, 256, 0, g, (const double*)P.x64, P.ei.k3, P.ei.k2, (const double*)P.dK0b,
              P.ei.wht ? 1 : 0, (double*)nullptr, (const double*)P.rho_f, P.gsens, penalty, void_);
-      launch(P, k_filter_T, nbe, 256, 0, F.g, F.taps, (const double*)F.N, (const double*)P.gsens, P.it_dr_new);
+      P.nlaunch += filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, P.it_dr_new, P.stream);
+      KCHECK();
     }
     n_fixed1 = P.nlaunch - c0;
   });
@@ -3195,7 +3200,8 @@ int edge_filter_create(int dim, const int* nel, int n_taps, const int* offsets, 
     delete f;
     fail(EDGE_ECUDA, cudaGetErrorString(e));
   }
-  k_filter_norm<<<cdiv(f->n_el, 256), 256>>>(f->g, f->taps, f->N);
+  f->tiled = make_tap_cols(dim, f->taps, f->cols);
+  filter_norm(f->g, f->taps, f->N, nullptr);
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     delete f;
@@ -3214,7 +3220,8 @@ int edge_filter_destroy(edge_filter* f) {
 int edge_filter_apply(edge_filter* f, const double* in_dev, double* out_dev, void* stream) {
   API_BEGIN
   if (!f || !in_dev || !out_dev) fail(EDGE_EINVAL, "null argument");
-  k_filter<<<cdiv(f->n_el, 256), 256, 0, (cudaStream_t)stream>>>(f->g, f->taps, in_dev, out_dev);
+  filter_forward(f->g, f->taps, f->tile(), f->N, in_dev, FilterOut{out_dev, nullptr, nullptr, 0.0, 0.0, f->g},
+                 (cudaStream_t)stream);
   KCHECK();
   API_END
 }
@@ -3222,7 +3229,7 @@ int edge_filter_apply(edge_filter* f, const double* in_dev, double* out_dev, voi
 int edge_filter_apply_T(edge_filter* f, const double* in_dev, double* out_dev, void* stream) {
   API_BEGIN
   if (!f || !in_dev || !out_dev) fail(EDGE_EINVAL, "null argument");
-  k_filter_T<<<cdiv(f->n_el, 256), 256, 0, (cudaStream_t)stream>>>(f->g, f->taps, f->N, in_dev, out_dev);
+  filter_transpose(f->g, f->taps, f->tile(), f->N, in_dev, out_dev, (cudaStream_t)stream);
   KCHECK();
   API_END
 }
@@ -3575,7 +3582,8 @@ int edge_simp_solve_and_process(edge_problem* p, edge_filter* f, const double* r
   double* rf = rho_f_dev ? rho_f_dev : P.rho_f;
   const unsigned nbe = cdiv(P.n_el, 256);
   // rho_f = H rho ; E = clip(rho_f^p, void, 1)
-  launch(P, k_filter_material<double, float>, nbe, 256, 0, g, f->taps, rho_dev, rf, P.E64, P.E32, penalty, void_, 0);
+  P.nlaunch += filter_forward(f->g, f->taps, f->tile(), f->N, rho_dev, FilterOut{rf, P.E64, P.E32, penalty, void_, g},
+                              P.stream);
   KCHECK();
   P.has_rho = true;
   // U = K(E)^-1 f (warm start from U_dev)
@@ -3593,7 +3601,7 @@ int edge_simp_solve_and_process(edge_problem* p, edge_filter* f, const double* r
   // dr = H^T (p clip(rho_f)^(p-1) dk)
   launch(P, k_dk<double>, nbe, 256, 0, g, P.x64, P.ei.k3, P.ei.k2, P.dK0b, P.ei.wht ? 1 : 0, nullptr, rf, P.gsens,
                                           penalty, void_);
-  launch(P, k_filter_T, nbe, 256, 0, f->g, f->taps, f->N, P.gsens, dr_dev);
+  P.nlaunch += filter_transpose(f->g, f->taps, f->tile(), f->N, P.gsens, dr_dev, P.stream);
   launch(P, k_slots_to_user<double>, cdiv(g.n, 256), 256, 0, g, P.x64, U_dev);
   KCHECK();
   CK(cudaMemcpyAsync(P.scal_h + 2, P.scal + 2, sizeof(double), cudaMemcpyDeviceToHost, P.stream));
@@ -3972,9 +3980,9 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
       Geo gr = g;  // the real grid's extents in the problem's slot layout
       gr.nx = B.nxr[i];
       gr.ny = B.nyr[i];
-      const unsigned nbe = cdiv(F.n_el, 256);
-      launch(P, k_filter_material<double, float>, nbe, 256, 0, gr, F.taps, rho[i], P.rho_f, P.E64, P.E32, penalty,
-             void_, 0);
+      P.nlaunch += filter_forward(F.g, F.taps, F.tile(), F.N, rho[i],
+                                  FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, gr}, P.stream);
+      KCHECK();
       P.has_rho = true;
       launch(P, k_user_to_slots_pad, cdiv(g.n, 256), 256, 0, g, B.nxr[i], B.nyr[i], f[i], P.b64);
       if (use_last)
@@ -4069,7 +4077,8 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
              (const double*)P.x64, P.part, P.ticket, P.scal + 2);
       launch(P, k_dk<double>, nbe, 256, 0, gr, (const double*)P.x64, P.ei.k3, P.ei.k2, (const double*)P.dK0b,
              P.ei.wht ? 1 : 0, (double*)nullptr, (const double*)P.rho_f, P.gsens, penalty, void_);
-      launch(P, k_filter_T, nbe, 256, 0, F.g, F.taps, (const double*)F.N, (const double*)P.gsens, dr[i]);
+      P.nlaunch += filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, dr[i], P.stream);
+      KCHECK();
       launch(P, k_slots_to_user_pad, cdiv(g.n, 256), 256, 0, g, B.nxr[i], B.nyr[i], (const double*)P.x64, U[i]);
     } catch (...) {
       P.stream = saved;

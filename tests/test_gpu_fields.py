@@ -31,3 +31,33 @@ def test_oc_update_equals_sequential_bisection(n, vf):
     assert (lo.value, so.value) == (lam, steps)
     np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=4e-16, atol=0)
     assert ch.value == pytest.approx(float(((ref - rho) ** 2).sum()), rel=1e-12)
+
+
+@pytest.mark.parametrize("nel", [(1, 1), (31, 33), (32, 32), (70, 65), (1, 1, 1), (3, 2, 5), (4, 16, 32), (5, 17, 33),
+                                 (9, 40, 31)])
+@pytest.mark.parametrize("rmin", [1.0, 1.5, 2.0, 2.9, 5.5])
+def test_filter_and_transpose_against_taps(nel, rmin):
+    """H and H^T against the tap sums in numpy, where tiles end and at every halo width (5.5: the
+    one-thread-per-element kernel, 2-D only).  At most 128 terms of order 1 per sum, whose weights add
+    to 1: a few FP64 roundings."""
+    import torch
+    import edge_to_b200 as eb
+    dim = len(nel)
+    if rmin > 3.0 and dim == 3:
+        pytest.skip("more taps than the filter takes")
+    mesh = (eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D)(*nel, *map(float, nel))
+    flt = (eb.CuStructuredFilter2D if dim == 2 else eb.CuStructuredFilter3D)(mesh, rmin)
+    rng = np.random.default_rng(7)
+    x, y = rng.uniform(size=nel), rng.standard_normal(nel)
+    offs, w = flt.offsets.cpu().numpy(), flt.weights.cpu().numpy()
+    idx = np.stack(np.meshgrid(*[np.arange(n) for n in nel], indexing="ij"), -1).reshape(-1, dim)
+    H = np.zeros((idx.shape[0], idx.shape[0]))
+    for o, wk in zip(offs, w):
+        nb = idx + o
+        ok = np.all((nb >= 0) & (nb < np.array(nel)), axis=1)
+        H[np.nonzero(ok)[0], np.ravel_multi_index(nb[ok].T, nel)] += wk
+    H /= H.sum(axis=1, keepdims=True)
+    fx = flt.dot(torch.as_tensor(x.ravel(), device="cuda")).cpu().numpy()
+    ty = flt.T.dot(torch.as_tensor(y.ravel(), device="cuda")).cpu().numpy()
+    np.testing.assert_allclose(fx, H @ x.ravel(), rtol=0, atol=2e-15)
+    np.testing.assert_allclose(ty, H.T @ y.ravel(), rtol=0, atol=2e-14)
