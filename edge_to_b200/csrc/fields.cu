@@ -796,4 +796,506 @@ int filter_norm(const Geo& g, const Taps& t, double* N, cudaStream_t stream) {
   return 1;
 }
 
+// ------------------------------------------------------------------ operator on user vectors, 2-D
+// K(E) u straight from and to the user's interleaved vectors: one launch instead of the conversion
+// to slots, the tiled product and the conversion back.  One thread per node gathers its nine
+// neighbours (16-byte pairs where the vector is 16-byte aligned; a neighbour outside the grid reads
+// the node itself and counts as zero, so that all loads of a thread are in flight together) and the
+// four surrounding elements, 64 FMA with the element matrix in the constant bank.  What bounds it
+// is the launch and two round trips to L2: at 131,841 nodes the FMA take 0.5 us.
+template <bool PAIR> EDGE_D double2 user_pair(const double* __restrict__ u, long long node) {
+  if constexpr (PAIR) return __ldg(reinterpret_cast<const double2*>(u) + node);
+  else return make_double2(__ldg(u + 2 * node), __ldg(u + 2 * node + 1));
+}
+template <bool PAIR>
+__global__ void __launch_bounds__(128)
+k_product2_user(const Geo g, const __grid_constant__ K2Dense K, const double* __restrict__ E,
+                const uint8_t* __restrict__ mask, const double* __restrict__ u, double* __restrict__ out) {
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 4 + (threadIdx.x >> 5);
+  if (i >= g.nx || j >= g.ny) return;
+  const long long node = (long long)j * g.nx + i, s = g.slot2(i, j);
+  double U[3][3][2], Ee[2][2];
+  double2 raw = make_double2(0.0, 0.0);
+  unsigned mc = 0;
+#pragma unroll
+  for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+    for (int dx = -1; dx <= 1; ++dx) {
+      const bool in = i + dx >= 0 && i + dx < g.nx && j + dy >= 0 && j + dy < g.ny;
+      const double2 v = user_pair<PAIR>(u, in ? node + (long long)dy * g.nx + dx : node);
+      const unsigned m = in ? __ldg(mask + s + (long long)dy * g.pz + dx) : 3u;
+      if (dx == 0 && dy == 0) {
+        raw = v;
+        mc = m;
+      }
+      U[dy + 1][dx + 1][0] = (m & 1) ? 0.0 : v.x;
+      U[dy + 1][dx + 1][1] = (m & 2) ? 0.0 : v.y;
+    }
+#pragma unroll
+  for (int ay = 0; ay < 2; ++ay)
+#pragma unroll
+    for (int ax = 0; ax < 2; ++ax) {  // the element of which the node is corner (ax, ay)
+      const int li = i - ax, lj = j - ay;
+      const bool ev = li >= 0 && lj >= 0 && li < g.nx - 1 && lj < g.ny - 1;
+      const double x = __ldg(E + (ev ? g.slot2(li, lj) : s));
+      Ee[ay][ax] = ev ? x : 0.0;
+    }
+  double A0 = 0.0, A1 = 0.0;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int ax = a & 1, ay = a >> 1;
+    double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        const double ub = U[(b >> 1) - ay + 1][(b & 1) - ax + 1][d];
+        r0 = fma(K.k[(a * 2 + 0) * 8 + b * 2 + d], ub, r0);
+        r1 = fma(K.k[(a * 2 + 1) * 8 + b * 2 + d], ub, r1);
+      }
+    A0 = fma(Ee[ay][ax], r0, A0);
+    A1 = fma(Ee[ay][ax], r1, A1);
+  }
+  if (mc & 1) A0 = raw.x;
+  if (mc & 2) A1 = raw.y;
+  if constexpr (PAIR) {
+    reinterpret_cast<double2*>(out)[node] = make_double2(A0, A1);
+  } else {
+    out[2 * node] = A0;
+    out[2 * node + 1] = A1;
+  }
+}
+
+// Element energies: elements run along y in the reference's order, nodes along x, so a block stages
+// the 33 x 33 nodes of 32 x 32 elements (rows along x, coalesced) and its lanes then walk elements
+// along y (coalesced stores; the row pitch of 33 pairs keeps eight lanes on different banks).
+EDGE_D double energy2(const KHat2<double>& K, const double u[4][2]) { return elem2_energy(K, u); }
+EDGE_D double energy2(const K2Dense& K, const double u[4][2]) {
+  double acc = 0.0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t += K.k[r * 8 + q] * u[q >> 1][q & 1];
+    acc += u[r >> 1][r & 1] * t;
+  }
+  return acc;
+}
+template <bool PAIR, class K2>
+__global__ void __launch_bounds__(256)
+k_energy2_user(const Geo g, const __grid_constant__ K2 K, const double* __restrict__ u, double* __restrict__ dk) {
+  __shared__ double2 sh[33 * 33];
+  const int nelx = g.nx - 1, nely = g.ny - 1;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+  constexpr int U = 5;  // 33 * 33 nodes over 256 threads
+  double2 v[U];
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int q = threadIdx.x + k * 256, i = x0 + q % 33, j = y0 + q / 33;
+    const bool in = q < 33 * 33 && i < g.nx && j < g.ny;
+    v[k] = in ? user_pair<PAIR>(u, (long long)j * g.nx + i) : make_double2(0.0, 0.0);
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (threadIdx.x + k * 256 < 33 * 33) sh[threadIdx.x + k * 256] = v[k];
+  __syncthreads();
+  const int ly = threadIdx.x & 31, j = y0 + ly;
+  if (j >= nely) return;
+  for (int lx = threadIdx.x >> 5; lx < 32; lx += 8) {
+    const int i = x0 + lx;
+    if (i >= nelx) break;
+    double ue[4][2];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const double2 p = sh[(ly + (b >> 1)) * 33 + lx + (b & 1)];
+      ue[b][0] = p.x;
+      ue[b][1] = p.y;
+    }
+    dk[(long long)i * nely + j] = -energy2(K, ue);
+  }
+}
+
+static bool pair_aligned(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+int product2_user(const Geo& g, const K2Dense& K, const double* E, const uint8_t* mask, const double* u, double* out,
+                  cudaStream_t stream) {
+  const dim3 grid((g.nx + 31) / 32, (g.ny + 3) / 4);
+  if (pair_aligned(u) && pair_aligned(out))
+    k_product2_user<true><<<grid, 128, 0, stream>>>(g, K, E, mask, u, out);
+  else
+    k_product2_user<false><<<grid, 128, 0, stream>>>(g, K, E, mask, u, out);
+  return 1;
+}
+template <class K2>
+static int energy2_launch(const Geo& g, const K2& K, const double* u, double* dk, cudaStream_t stream) {
+  const dim3 grid((g.nx - 1 + 31) / 32, (g.ny - 1 + 31) / 32);
+  if (pair_aligned(u))
+    k_energy2_user<true, K2><<<grid, 256, 0, stream>>>(g, K, u, dk);
+  else
+    k_energy2_user<false, K2><<<grid, 256, 0, stream>>>(g, K, u, dk);
+  return 1;
+}
+int energy2_user(const Geo& g, const K2Dense& K, const KHat2<double>* box, const double* u, double* dk,
+                 cudaStream_t stream) {
+  return box ? energy2_launch(g, *box, u, dk, stream) : energy2_launch(g, K, u, dk, stream);
+}
+
+// ------------------------------------------------------------------ operator on user vectors, 3-D
+// K(E) u (or the element energies u_e^T K0 u_e) straight from the user's interleaved vector, FP64.
+// The walk is the one of the TMA kernel (fine_tma.cuh): 8 warps of 16 z-lanes x 2 x-columns march
+// along y with one element per thread and layer, in the Walsh transform domain.  A user row (3 nz
+// doubles) has no 16-byte pitch, so planes arrive by 8-byte cp.async copies into a four-stage ring
+// (zero-filled outside the grid), each thread copying the same four positions of every plane; E and the
+// constraint flags of a layer are fetched one layer ahead.  The in-plane sums of neighbouring warps
+// are exchanged through shared memory and picked up one layer later, so that a layer has one
+// barrier; outputs are gathered per warp and stored contiguously.
+//
+// Layers are unrolled by four: stages are constants and the lower and upper plane swap without copies
+// (103M warp instructions at 12.8M DOF rolled, 61M unrolled).
+//
+// What bounds it: FP64 latency at 12 warps per SM.  An element takes 150 FP64 operations (200 without
+// the cube's block form): 45 us of the FP64 pipe at 12.8M DOF with the tiles' overlap, 37 us for the
+// bytes; it runs in 134.  Blocks of 4 warps at 168 registers, three per SM, measured best: 8 warps at
+// 128 registers 144 us (spills), four blocks 152 (spills), two 167.  The three launches it replaces
+// (user to slots, TMA product, slots to user) took 205 us.
+constexpr int U3_BX = 4, U3_NS = 4;
+constexpr int U3_NC = 2 * U3_BX, U3_NR = U3_NC + 1, U3_ROW = 51;  // element columns, node rows, doubles per row
+constexpr int U3_PLANE = U3_NR * U3_ROW, U3_PER = (U3_PLANE + 127) / 128;
+
+EDGE_D void cp_async8(void* dst, const void* src, bool valid) {
+  const int n = valid ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(n)
+               : "memory");
+}
+EDGE_D void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> EDGE_D void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// v = E Khat u for h = 1..7 (h = 0 is neither read nor written).
+EDGE_D void khat3(const KHat3<double>& K, double E, const double u[8][3], double v[8][3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int h = 1; h < 8; ++h) {
+      double a = K.dg[c][h] * u[h][c];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (d != c && (((h >> c) & 1) != ((h >> d) & 1))) a = fma(K.of[c][d][h], u[h ^ (1 << c) ^ (1 << d)][d], a);
+      v[h][c] = a * E;
+    }
+}
+EDGE_D void khat3(const KCube64& k, double E, const double u[8][3], double v[8][3]) {
+  const double nd = k.nd * E, no = k.no * E, sh = k.sh * E, bd = k.bd * E, bo = k.bo * E, td = k.td * E, to = k.to * E,
+               h7 = k.h7 * E;
+  const double ns = no * (u[1][0] + u[2][1] + u[4][2]);  // normal strains
+  v[1][0] = fma(nd, u[1][0], ns);
+  v[2][1] = fma(nd, u[2][1], ns);
+  v[4][2] = fma(nd, u[4][2], ns);
+  const double ts = to * (u[3][2] + u[5][1] + u[6][0]);  // twists
+  v[3][2] = fma(td, u[3][2], ts);
+  v[5][1] = fma(td, u[5][1], ts);
+  v[6][0] = fma(td, u[6][0], ts);
+  v[1][1] = v[2][0] = sh * (u[1][1] + u[2][0]);  // shears
+  v[1][2] = v[4][0] = sh * (u[1][2] + u[4][0]);
+  v[2][2] = v[4][1] = sh * (u[2][2] + u[4][1]);
+  v[3][0] = fma(bd, u[3][0], bo * u[6][2]);  // bending pairs
+  v[6][2] = fma(bd, u[6][2], bo * u[3][0]);
+  v[3][1] = fma(bd, u[3][1], bo * u[5][2]);
+  v[5][2] = fma(bd, u[5][2], bo * u[3][1]);
+  v[5][0] = fma(bd, u[5][0], bo * u[6][1]);
+  v[6][1] = fma(bd, u[6][1], bo * u[5][0]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v[7][c] = h7 * u[7][c];
+}
+EDGE_D void wht_plane(double t[2][2][3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const double p = t[b][0][c], q = t[b][1][c];
+      t[b][0][c] = p + q;
+      t[b][1][c] = p - q;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double p = t[0][h][c], q = t[1][h][c];
+      t[0][h][c] = p + q;
+      t[1][h][c] = p - q;
+    }
+  }
+}
+
+template <bool PRODUCT, class K3>
+__global__ void __launch_bounds__(32 * U3_BX, 3)
+k_user3(const Geo g, const __grid_constant__ K3 K, const double* __restrict__ E, const uint8_t* __restrict__ mask,
+        const uint8_t* __restrict__ eflag16, const int mpz, const int ly, const double* __restrict__ u,
+        double* __restrict__ out) {
+  __shared__ double sP[U3_NS][U3_PLANE];
+  __shared__ double sX[PRODUCT ? 2 : 1][PRODUCT ? U3_BX : 1][16][3];
+  __shared__ double sO[PRODUCT ? U3_BX : 1][2][48];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int zl = lane & 15, xh = lane >> 4, cx = 2 * w + xh;
+  // first node column / z of the tile: one before the outputs for the product
+  const int tz = PRODUCT ? (int)blockIdx.x * 15 - 1 : (int)blockIdx.x * 16;
+  const int tx = PRODUCT ? (int)blockIdx.y * (U3_NC - 1) - 1 : (int)blockIdx.y * U3_NC;
+  const int rows = PRODUCT ? g.ny : g.ny - 1;  // output planes / element rows
+  const int y0 = blockIdx.z * ly, y1 = min(y0 + ly, rows);
+  const int p0 = PRODUCT ? y0 - 1 : y0, np = y1 - p0 + 1;
+  const int ez = tz + zl, ex = tx + cx;
+
+  // the positions of a plane that this thread copies, as one pointer that moves a plane per copy
+  int off[U3_PER];
+  bool ok[U3_PER];
+#pragma unroll
+  for (int t = 0; t < U3_PER; ++t) {
+    const int q = threadIdx.x + t * (32 * U3_BX), r = q / U3_ROW, c = q % U3_ROW;
+    const int x = tx + r, z = tz + c / 3;
+    ok[t] = q < U3_PLANE && x >= 0 && x < g.nx && z >= 0 && z < g.nz;
+    off[t] = ok[t] ? (x * g.nz + z) * 3 + c % 3 : 0;
+  }
+  const long long pl = 3LL * g.nx * g.nz;
+  const double* src = u + p0 * pl;  // plane p0 + (next k); dereferenced only inside the grid
+  int pk = p0;
+  auto issue = [&](int stage) {
+    const bool in = pk >= 0 && pk < g.ny && pk <= y1;
+    const double* from = in ? src : u;
+#pragma unroll
+    for (int t = 0; t < U3_PER; ++t)
+      if (t + 1 < U3_PER || threadIdx.x + t * (32 * U3_BX) < U3_PLANE)
+        cp_async8(sP[stage] + threadIdx.x + t * (32 * U3_BX), from + off[t], in && ok[t]);
+    cp_commit();
+    src += pl;
+    ++pk;
+  };
+  const bool col = ex >= 0 && ex < g.nx && ez >= 0 && ez < g.nz;
+  // E and the constraint flag of this thread's column, one plane of slots per step
+  const double* Ep = PRODUCT && col ? E + g.slot3(ex, 0, ez) : nullptr;
+  const uint8_t* Fp = PRODUCT && col ? eflag16 + (long long)ex * mpz + ez : nullptr;
+  const long long fpl = (long long)g.nx * mpz;
+  auto elem_E = [&](int ey) -> double { return col && (unsigned)ey < (unsigned)g.ny ? __ldg(Ep + ey * g.plane) : 0.0; };
+  auto elem_flag = [&](int ey) -> unsigned {
+    return col && (unsigned)ey < (unsigned)g.ny ? __ldg(Fp + ey * fpl) : 0u;
+  };
+  // constrained DOFs of the four corners on plane p read as zero (flagged columns: ex, ez >= 0)
+  auto mask_plane = [&](int p, double t[2][2][3]) {
+#pragma unroll
+    for (int dx = 0; dx < 2; ++dx)
+#pragma unroll
+      for (int dz = 0; dz < 2; ++dz)
+        if (ex + dx < g.nx && ez + dz < g.nz && p >= 0 && p < g.ny) {
+          const unsigned m = __ldg(mask + g.slot3(ex + dx, p, ez + dz));
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            if ((m >> c) & 1) t[dx][dz][c] = 0.0;
+        }
+  };
+  const double* corner = sP[0] + cx * U3_ROW + 3 * zl;
+  auto load_plane = [&](int stage, double t[2][2][3]) {
+#pragma unroll
+    for (int dx = 0; dx < 2; ++dx)
+#pragma unroll
+      for (int dz = 0; dz < 2; ++dz)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[dx][dz][c] = corner[stage * U3_PLANE + dx * U3_ROW + 3 * dz + c];
+  };
+
+#pragma unroll
+  for (int k = 0; k < U3_NS - 1; ++k) issue(k);
+  // E and flags of the coming layers, fetched two layers before they are used
+  double Ee = PRODUCT ? elem_E(p0) : 1.0, E1 = PRODUCT ? elem_E(p0 + 1) : 1.0;
+  unsigned fl = PRODUCT ? elem_flag(p0) : 0u, fn = PRODUCT ? elem_flag(p0 + 1) : 0u, f2 = PRODUCT ? elem_flag(p0 + 2) : 0u;
+  cp_wait<U3_NS - 2>();
+  __syncthreads();
+  double pa[2][2][3], pb[2][2][3], car[2][2][3], pend[3];
+  load_plane(0, pa);
+  if (PRODUCT && fl) mask_plane(p0, pa);
+  wht_plane(pa);
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) car[a][b][c] = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) pend[c] = 0.0;
+  unsigned pfl = 0;
+  // this lane's three places of the warp half's output row (16 nodes from z = tz), moving a plane per
+  // store
+  bool st[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const int d = zl + 16 * t;
+    st[t] = PRODUCT && cx >= 1 && ex < g.nx && d >= 3 && tz + d / 3 < g.nz;
+  }
+  double* op = out + (((long long)y0 * g.nx + ex) * g.nz + tz) * 3 + zl;  // dereferenced only where st
+
+  // completes and stores plane p, the output of the layer before; X: its exchange buffer
+  auto flush = [&](int p, int X) {
+    double a[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a[c] = pend[c];
+    if (xh == 0 && w > 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a[c] += sX[X][w - 1][zl][c];
+    }
+    if (pfl && zl >= 1 && cx >= 1) {  // identity rows
+      const unsigned m = __ldg(mask + g.slot3(ex, p, ez));
+      const long long node = ((long long)p * g.nx + ex) * g.nz + ez;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if ((m >> c) & 1) a[c] = __ldg(u + 3 * node + c);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sO[w][xh][3 * zl + c] = a[c];
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+      if (st[t]) op[16 * t] = sO[w][xh][zl + 16 * t];
+    op += pl;
+  };
+
+  // one layer: element row ey between the planes lo (transformed) and the one in stage S
+  auto layer = [&](int ey, auto stage, double lo[2][2][3], double hi[2][2][3]) {
+    constexpr int S = decltype(stage)::value;  // the new plane's stage = (layer + 1) mod 4
+    cp_wait<U3_NS - 3>();
+    __syncthreads();
+    issue((S + U3_NS - 2) % U3_NS);
+    double E2 = 1.0;
+    unsigned f3 = 0u;
+    if constexpr (PRODUCT) {
+      E2 = elem_E(ey + 2);
+      f3 = elem_flag(ey + 3);
+      if (ey > y0) flush(ey - 1, S & 1);
+    }
+    load_plane(S, hi);
+    // the new plane is also the lower face of the next element row: masked by both rows' flags
+    if (PRODUCT && (fl | fn)) mask_plane(ey + 1, hi);
+    wht_plane(hi);
+    double uh[8][3], vh[8][3];
+#pragma unroll
+    for (int hx = 0; hx < 2; ++hx)
+#pragma unroll
+      for (int hz = 0; hz < 2; ++hz)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (hx | hz) uh[hx | (hz << 2)][c] = lo[hx][hz][c] + hi[hx][hz][c];
+          uh[hx | 2 | (hz << 2)][c] = lo[hx][hz][c] - hi[hx][hz][c];
+        }
+    khat3(K, Ee, uh, vh);
+    if constexpr (PRODUCT) {
+      double cur[2][2][3];
+#pragma unroll
+      for (int hx = 0; hx < 2; ++hx)
+#pragma unroll
+        for (int hz = 0; hz < 2; ++hz)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double b = vh[hx | 2 | (hz << 2)][c];
+            if (hx | hz) {
+              const double a = vh[hx | (hz << 2)][c];
+              cur[hx][hz][c] = car[hx][hz][c] + (a + b);
+              car[hx][hz][c] = a - b;
+            } else {  // transform coefficient 0 vanishes
+              cur[0][0][c] = car[0][0][c] + b;
+              car[0][0][c] = -b;
+            }
+          }
+      wht_plane(cur);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double g0 = cur[0][0][c] + __shfl_up_sync(0xffffffffu, cur[0][1][c], 1, 16);
+        const double g1 = cur[1][0][c] + __shfl_up_sync(0xffffffffu, cur[1][1][c], 1, 16);
+        const double fromL = __shfl_up_sync(0xffffffffu, g1, 16);
+        pend[c] = xh ? g0 + fromL : g0;
+        if (xh) sX[(S + 1) & 1][w][zl][c] = g1;
+      }
+      pfl = fl;
+    } else {
+      double e = 0.0;
+#pragma unroll
+      for (int h = 1; h < 8; ++h)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) e = fma(uh[h][c], vh[h][c], e);
+      if (ex < g.nx - 1 && ez < g.nz - 1) out[((long long)ex * (g.ny - 1) + ey) * (g.nz - 1) + ez] = -e;
+    }
+    Ee = E1;
+    E1 = E2;
+    fl = fn;
+    fn = f2;
+    f2 = f3;
+  };
+  // layers in groups of four: the stage is then a constant and the two planes swap without copies
+  int ey = p0;
+  const int last = p0 + np - 1;  // one past the last element row
+  int done = 0;
+  for (; ey + 4 <= last; ey += 4) {
+    layer(ey, std::integral_constant<int, 1>{}, pa, pb);
+    layer(ey + 1, std::integral_constant<int, 2>{}, pb, pa);
+    layer(ey + 2, std::integral_constant<int, 3>{}, pa, pb);
+    layer(ey + 3, std::integral_constant<int, 0>{}, pb, pa);
+  }
+  if (ey < last) {
+    layer(ey, std::integral_constant<int, 1>{}, pa, pb);
+    done = 1;
+  }
+  if (ey + 1 < last) {
+    layer(ey + 1, std::integral_constant<int, 2>{}, pb, pa);
+    done = 2;
+  }
+  if (ey + 2 < last) {
+    layer(ey + 2, std::integral_constant<int, 3>{}, pa, pb);
+    done = 3;
+  }
+  if constexpr (PRODUCT) {
+    __syncthreads();
+    flush(last - 1, (done + 1) & 1);  // the last layer wrote buffer (its stage + 1) & 1
+  }
+  cp_wait<0>();
+}
+
+// Planes per block: the number of y-chunks that needs the fewest layers in all, counting the waves of
+// 2 x 148 resident blocks and one and a half layers of start-up per block.
+static int user3_chunk(long long tiles, int rows) {
+  long long best = -1;
+  int best_ly = rows;
+  for (int c = 1; c <= rows && c <= 4096; ++c) {
+    const int ly = (rows + c - 1) / c;
+    const long long blocks = tiles * ((rows + ly - 1) / ly);
+    const long long cost = ((blocks + 443) / 444) * (2LL * ly + 3);
+    if (best < 0 || cost < best) {
+      best = cost;
+      best_ly = ly;
+    }
+    if (tiles * c > 444LL * 64) break;
+  }
+  return best_ly;
+}
+
+bool user_grid_ok(const Geo& g) {
+  if (g.dim == 2) return (g.ny + 3) / 4 <= 65535;
+  return 3LL * g.nx * g.nz < (1LL << 31) && (g.nx + 14) / 15 <= 65535 && g.ny <= 65535;
+}
+
+template <bool PRODUCT, class K3>
+static int user3_launch(const Geo& g, const K3& K, const double* E, const uint8_t* mask, const uint8_t* eflag16, int mpz,
+                        const double* u, double* out, cudaStream_t stream) {
+  const int step = PRODUCT ? 15 : 16, sx = PRODUCT ? U3_NC - 1 : U3_NC, nz = PRODUCT ? g.nz : g.nz - 1, nx = PRODUCT ? g.nx : g.nx - 1;
+  const int rows = PRODUCT ? g.ny : g.ny - 1;
+  const unsigned tz = (unsigned)((nz + step - 1) / step), tx = (unsigned)((nx + sx - 1) / sx);
+  const int ly = user3_chunk((long long)tz * tx, rows);
+  k_user3<PRODUCT, K3><<<dim3(tz, tx, (unsigned)((rows + ly - 1) / ly)), 32 * U3_BX, 0, stream>>>(g, K, E, mask, eflag16,
+                                                                                              mpz, ly, u, out);
+  return 1;
+}
+int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* E, const uint8_t* mask,
+                  const uint8_t* eflag16, int mpz, const double* u, double* out, cudaStream_t stream) {
+  if (cube) return user3_launch<true>(g, *cube, E, mask, eflag16, mpz, u, out, stream);
+  return user3_launch<true>(g, K, E, mask, eflag16, mpz, u, out, stream);
+}
+int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* u, double* dk,
+                 cudaStream_t stream) {
+  if (cube) return user3_launch<false>(g, *cube, nullptr, nullptr, nullptr, 0, u, dk, stream);
+  return user3_launch<false>(g, K, nullptr, nullptr, nullptr, 0, u, dk, stream);
+}
+
 }  // namespace edge

@@ -76,4 +76,30 @@ int filter_transpose(const Geo& g, const Taps& t, const TapCols* c, const double
                      cudaStream_t stream);
 int filter_norm(const Geo& g, const Taps& t, double* N, cudaStream_t stream);
 
+// ------------------------------------------------------------------ operator on user vectors
+// Element matrix of a 2-D problem, corner-bit order, row-major.
+struct K2Dense {
+  double k[64];
+};
+// out = K(E) u with identity rows on constrained DOFs, u and out in the user's layout
+// (v[2 node + c], node = j nx + i); E and mask in the slots of g.
+int product2_user(const Geo& g, const K2Dense& K, const double* E, const uint8_t* mask, const double* u, double* out,
+                  cudaStream_t stream);
+// dk_e = -u_e^T K0 u_e per element (reference element order) from a user-layout displacement; box: the
+// transformed element matrix when it has the box structure, else null
+int energy2_user(const Geo& g, const K2Dense& K, const KHat2<double>* box, const double* u, double* dk,
+                 cudaStream_t stream);
+
+// The same in 3-D, for element matrices with the box structure (KHat3, element_op.cuh) and, when
+// `cube` is given, its block form (equal edges, isotropic material: KCube64).
+struct KCube64 {
+  double nd, no, sh, bd, bo, td, to, h7;  // nd and td without the shared part no / to
+};
+int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* E, const uint8_t* mask,
+                  const uint8_t* eflag16, int mpz, const double* u, double* out, cudaStream_t stream);
+int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* u, double* dk,
+                 cudaStream_t stream);
+// Grids that the launches above take (their tile counts are grid dimensions).
+bool user_grid_ok(const Geo& g);
+
 }  // namespace edge

@@ -225,6 +225,8 @@ struct Prob {
   KHat3P k3p;              // packed transformed element operator (FP32 pairs)
   KCube kcube;             // block form of the same operator (cube elements)
   bool cube = false;       // kcube reproduces every entry of the transformed operator
+  KCube64 kcube64;         // the same in FP64
+  bool cube64 = false;     // ... to FP64 rounding
   int blocks_per_sm = 4;   // y-chunking target of the fine kernel
   // per kind of fused cube launch (0: first sweep + residual, 1: last sweep + correction,
   // 2: search direction + product), the tile variant and y-chunking target chosen for that
@@ -552,7 +554,9 @@ static KHat3P pack3(const KHat3<double>& k) {
 
 // Block form of a cube element's transformed operator (fine_cube.cuh): read the eight
 // coefficients off KHat3 and accept them only if the model reproduces all 576 entries.
-static bool cube_form(const KHat3<double>& k, KCube& out) {
+// out64: the same in FP64, valid (*ok64) when the entries agree to rounding.
+static bool cube_form(const KHat3<double>& k, KCube& out, KCube64& out64, bool& ok64) {
+  ok64 = false;
   const double nd = k.dg[0][1], no = k.of[0][1][1], sh = k.dg[1][1], bd = k.dg[0][3], bo = k.of[0][2][3],
                td = k.dg[2][3], to = k.of[2][1][3], h7 = k.dg[0][7];
   // model entries: M[(h,c)][(h2,c2)]
@@ -590,6 +594,8 @@ static bool cube_form(const KHat3<double>& k, KCube& out) {
           dev = std::max(dev, std::fabs(a - M[h][c][h2][c2]));
         }
   if (!(mx > 0.0) || dev > 1e-12 * mx) return false;
+  out64 = KCube64{nd - no, no, sh, bd, bo, td - to, to, h7};
+  ok64 = dev <= 1e-15 * mx;
   out = KCube{(float)(nd - no), (float)no, (float)sh, (float)bd, (float)bo, (float)(td - to), (float)to, (float)h7};
   return true;
 }
@@ -2222,7 +2228,7 @@ int edge_problem_create(int dim, const int* nel, const double* K0, int precision
     analyse_element(dim, K0, P.ei);
     if (dim == 3) {
       P.k3p = pack3(P.ei.k3);
-      P.cube = P.ei.wht && cube_form(P.ei.k3, P.kcube);
+      P.cube = P.ei.wht && cube_form(P.ei.k3, P.kcube, P.kcube64, P.cube64);
     }
     const int nk = P.ei.nk;
     P.dK0b = P.alloc<double>(nk * nk);
@@ -2707,12 +2713,34 @@ int edge_mg_solve_embedded(edge_problem* p, const int* nel_real, const double* f
   API_END
 }
 
+// Whether two arrays of doubles share memory (kernel.dot(kernel.dot(u)) hands its own result back).
+static bool overlap(const double* a, long long na, const double* b, long long nb) {
+  return (uintptr_t)a < (uintptr_t)(b + nb) && (uintptr_t)b < (uintptr_t)(a + na);
+}
+static K2Dense k2_dense(const Prob& P) {
+  K2Dense K;
+  std::copy(P.ei.K0b, P.ei.K0b + 64, K.k);
+  return K;
+}
+
 int edge_matvec(edge_problem* p, const double* u_dev, double* out_dev) {
   API_BEGIN
   if (!p || !u_dev || !out_dev) fail(EDGE_EINVAL, "null argument");
   Prob& P = p->P;
   if (!P.has_rho) fail(EDGE_ESTATE, "Rho has not been set. dot works only after setting rho.");
   const Geo& g = P.g0;
+  // one launch on the user's vectors; with springs, an element matrix without the box structure, the TMA
+  // switch off or a result over its own input, the solver's operator between two conversions
+  if (P.n_springs == 0 && user_grid_ok(g) && (P.dim == 2 || (P.ei.wht && P.use_tma)) &&
+      !overlap(u_dev, P.n_dof, out_dev, P.n_dof)) {
+    if (P.dim == 2)
+      P.nlaunch += product2_user(g, k2_dense(P), P.E64, P.mask, u_dev, out_dev, P.stream);
+    else
+      P.nlaunch += product3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.E64, P.mask, P.eflag16, P.mpz, u_dev,
+                                 out_dev, P.stream);
+    KCHECK();
+    return EDGE_OK;
+  }
   launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, u_dev, P.b64);
   EpiStore<double, double> e{P.r64, g.n};
   fine_apply<double>(P, P.b64, e, nullptr);
@@ -2774,9 +2802,18 @@ int edge_process_grad(edge_problem* p, const double* U_dev, double* dk_dev) {
   if (!p || !U_dev || !dk_dev) fail(EDGE_EINVAL, "null argument");
   Prob& P = p->P;
   const Geo& g = P.g0;
-  launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, U_dev, P.b64);
-  launch(P, k_dk<double>, cdiv(P.n_el, 256), 256, 0, g, P.b64, P.ei.k3, P.ei.k2, P.dK0b, P.ei.wht ? 1 : 0, dk_dev,
-                                                         nullptr, nullptr, 0.0, 0.0);
+  // straight from the user's vector, unless the element matrix lacks the box structure (3-D) or the
+  // result lies over the input
+  if (user_grid_ok(g) && (P.dim == 2 || P.ei.wht) && !overlap(U_dev, P.n_dof, dk_dev, P.n_el)) {
+    if (P.dim == 2)
+      P.nlaunch += energy2_user(g, k2_dense(P), P.ei.wht ? &P.ei.k2 : nullptr, U_dev, dk_dev, P.stream);
+    else
+      P.nlaunch += energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, U_dev, dk_dev, P.stream);
+  } else {
+    launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, U_dev, P.b64);
+    launch(P, k_dk<double>, cdiv(P.n_el, 256), 256, 0, g, P.b64, P.ei.k3, P.ei.k2, P.dK0b, P.ei.wht ? 1 : 0, dk_dev,
+                                                           nullptr, nullptr, 0.0, 0.0);
+  }
   KCHECK();
   API_END
 }

@@ -61,3 +61,56 @@ def test_filter_and_transpose_against_taps(nel, rmin):
     ty = flt.T.dot(torch.as_tensor(y.ravel(), device="cuda")).cpu().numpy()
     np.testing.assert_allclose(fx, H @ x.ravel(), rtol=0, atol=2e-15)
     np.testing.assert_allclose(ty, H.T @ y.ravel(), rtol=0, atol=2e-14)
+
+
+def _problem(nel, seed, h=None):
+    import torch
+    import edge_to_b200 as eb
+    dim = len(nel)
+    h = h or [1.0] * dim
+    cls = eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D
+    mesh = cls(*nel, *[n * a for n, a in zip(nel, h)], stiffness=lambda x: eb.auto_stiffness(x, 1.0, 0.3))
+    k = eb.CuStructuredStiffnessKernel(mesh)
+    rng = np.random.default_rng(seed)
+    n_dof = int(np.prod([v + 1 for v in nel])) * dim
+    cons = rng.choice(n_dof, size=max(1, n_dof // 9), replace=False)
+    E = rng.uniform(1e-9, 1.0, int(np.prod(nel)))
+    u = rng.standard_normal(n_dof)
+    k.set_rho(torch.as_tensor(E, device="cuda"))
+    return mesh, k, cons, E, u
+
+
+def _dense(mesh, nel, E, u, cons):
+    """K(E) u and -u_e^T K0 u_e from the element matrix and the mesh's connectivity."""
+    dim = len(nel)
+    d = (np.asarray(mesh.elements)[:, :, None] * dim + np.arange(dim)).reshape(len(E), -1)
+    K0 = np.asarray(mesh.K_single)
+    v = u.copy()
+    v[cons] = 0.0
+    out = np.zeros_like(u)
+    np.add.at(out, d.ravel(), (E[:, None] * (v[d] @ K0)).ravel())
+    out[cons] = u[cons]
+    return out, -np.einsum("ei,ij,ej->e", u[d], K0, u[d])
+
+
+@pytest.mark.parametrize("nel", [(1, 1), (3, 4), (31, 3), (32, 33), (65, 130), (1, 1, 1), (2, 1, 3), (14, 5, 14), (15, 3, 15),
+                                 (16, 7, 31), (37, 40, 17)])
+@pytest.mark.parametrize("box", [False, True])
+def test_product_and_energy_on_user_vectors(nel, box):
+    """One-launch product and element energies where tiles end, on unit elements (the cube block form in
+    3-D) and on boxes, with and without constraints, on a vector that is only 8-byte aligned, and with
+    the product's own result as its input.  Entries of order 1 from at most 8 x 24 products of order
+    1: FP64 roundings of the sum, 1e-14."""
+    import torch
+    mesh, k, cons, E, u = _problem(nel, 11, [1.0, 1.5, 0.75][:len(nel)] if box else None)
+    ut = torch.as_tensor(u, device="cuda")
+    odd = torch.empty(u.size + 1, dtype=torch.float64, device="cuda")[1:]
+    odd.copy_(ut)
+    for c in (np.zeros(0, dtype=np.int64), cons):
+        k.set_constraints(c)
+        ref, dk = _dense(mesh, nel, E, u, c)
+        for x in (ut, odd):
+            np.testing.assert_allclose(k.dot(x).cpu().numpy(), ref, rtol=0, atol=3e-14)
+            np.testing.assert_allclose(k.process_grad(x).cpu().numpy(), dk, rtol=0, atol=1e-13)
+        twice, _ = _dense(mesh, nel, E, ref, c)
+        np.testing.assert_allclose(k.dot(k.dot(ut)).cpu().numpy(), twice, rtol=0, atol=2e-13)
