@@ -155,7 +155,9 @@ def check(code):
 
 
 def call(name, *args):
-    check(getattr(lib(), name)(*args))
+    rc = getattr(_lib or lib(), name)(*args)
+    if rc:
+        check(rc)
 
 
 def ptr(t):
@@ -178,6 +180,19 @@ def double_array(vals):
     return (ctypes.c_double * len(vals))(*[float(v) for v in vals])
 
 
+_raw_stream = None
+
+
 def stream_ptr():
-    import torch
-    return vp(torch.cuda.current_stream().cuda_stream)
+    """The current torch stream of the current device, as torch.cuda.current_stream() gives it, without
+    building its Stream object (3.4 us of a 10 us call)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.current_stream()  # initialises CUDA
+        raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        if raw is None or dev is None:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+        else:
+            _raw_stream = lambda: raw(dev())  # noqa: E731
+    return vp(_raw_stream())
