@@ -234,7 +234,7 @@ struct Prob {
   int kind_variant[3] = {-1, -1, -1};
   int kind_bps[3] = {0, 0, 0};
   bool kind_tune = true;  // edge_autotune_fine also picks the per-kind tiles
-  long long st_quad_max = 40000;   // 3-D stencil levels with at most this many slots use k_st3_apply_q
+  long long st_quad_max = 20000;   // 3-D stencil levels with at most this many slots use k_st3_apply_d
   bool st_bf16 = true;             // mixed precision: apply the coarse stencils from BF16 copies
   // mixed precision: the residual recurrence between FP64 replacements is stored in FP32
   // (arithmetic and r.r in FP64); false keeps an FP64 recurrence with an FP32 copy
@@ -965,7 +965,7 @@ template <typename T, class Epi, typename TS = T>
 static void st_apply(Prob& P, const Geo& g, const T* u, const TS* S, Epi epi, double* dot_dst) {
   CatScope cat(P, CAT_STENCIL);
   if (g.dim == 3 && g.n <= P.st_quad_max)
-    launch(P, k_st3_apply_q<T, TS, Epi>, dim3(cdiv(g.n * 4, 128)), dim3(128), 0, g, u, S, epi, P.part, P.ticket,
+    launch(P, k_st3_apply_d<T, TS, Epi>, dim3(cdiv(g.n, 32)), dim3(32 * ST3D_WARPS), 0, g, u, S, epi, P.part, P.ticket,
            dot_dst);
   else if (g.dim == 3 && P.st_pair && std::is_same<T, float>::value && g.n >= P.st_pair_min)
     launch(P, k_st3_apply2<T, TS, Epi>, dim3(cdiv(g.n / 2, 128)), dim3(128), 0, g, u, S, epi, P.part, P.ticket,

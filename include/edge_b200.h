@@ -153,7 +153,7 @@ int edge_set_graph(edge_problem* p, int enable);
 /* FP32 3-D coarse levels with at least min_slots slots use two nodes per thread (pair loads
  * of the centre and stored blocks; default 200000); min_slots < 0: one node per thread. */
 int edge_set_stencil_pair(edge_problem* p, long long min_slots);
-/* Mixed precision, 3-D: coarse levels (below the coarsest, above the four-lanes-per-node
+/* Mixed precision, 3-D: coarse levels (below the coarsest, above the warp-per-direction
  * size) with at least min_slots slots keep a tile-major BF16 pair copy of their stencil,
  * filled by every hierarchy set-up, and are applied from it two nodes per thread with
  * constant-offset coefficient loads and packed FP32 products (k_st3_apply2t); min_slots < 0:
@@ -181,9 +181,9 @@ int edge_set_residual32(edge_problem* p, int enable);
  * entry.  0 (default): plain stream order (at 12.8M DOF the SIMP loop ran 1.5 % faster so).
  * Host-driven solves always use plain order. */
 int edge_set_pdl(edge_problem* p, int enable);
-/* Coarse 3-D levels with at most max_slots slots use the four-lanes-per-node stencil kernel
- * (latency-bound small levels); larger levels one thread per node.  Default 40000 (at 70k
- * slots one thread per node is already faster). */
+/* Coarse 3-D levels with at most max_slots slots use the warp-per-direction stencil kernel
+ * (latency-bound small levels); larger levels one thread per node.  Default 20000 (at 38k nodes
+ * one thread per node is already as fast). */
 int edge_set_stencil_quad(edge_problem* p, long long max_slots);
 /* Benchmark helper: average device time (ms) of `reps` Jacobi sweeps of the stencil operator
  * on coarse level 1 <= level < n_level, in the problem's precision (hierarchy built). */
