@@ -1163,144 +1163,6 @@ __global__ void k_st_to_dense(const Geo g, const TS* __restrict__ S, double* __r
   }
 }
 
-// Blocked right-looking Cholesky (lower) of an SPD nd x nd row-major FP64 matrix, tile
-// size CB.  Per tile column K: k_chol_diag factors the diagonal tile in shared memory,
-// k_chol_panel solves the tiles below it, k_chol_update applies the symmetric rank-CB
-// update to the trailing lower triangle.  `status` is set to 1 on a non-positive pivot
-// (the pivot is then replaced by 1 so the factor stays finite).
-constexpr int CB = 32;
-
-__global__ void __launch_bounds__(CB * CB / 4) k_chol_diag(double* A, int nd, int K, int* status) {
-  EDGE_PDL_ENTRY();
-  __shared__ double t[CB][CB + 1];
-  const int k0 = K * CB;
-  const int m = min(CB, nd - k0);
-  for (int q = threadIdx.x; q < CB * CB; q += blockDim.x) {
-    const int r = q / CB, c = q % CB;
-    t[r][c] = (r < m && c < m) ? A[(long long)(k0 + r) * nd + k0 + c] : (r == c ? 1.0 : 0.0);
-  }
-  __syncthreads();
-  for (int k = 0; k < CB; ++k) {
-    if (threadIdx.x == 0) {
-      double d = t[k][k];
-      if (!(d > 0.0)) {
-        if (k < m) *status = 1;
-        d = 1.0;
-      }
-      t[k][k] = sqrt(d);
-    }
-    __syncthreads();
-    const double p = t[k][k];
-    for (int i = k + 1 + threadIdx.x; i < CB; i += blockDim.x) t[i][k] /= p;
-    __syncthreads();
-    for (int q = threadIdx.x; q < CB * CB; q += blockDim.x) {
-      const int i = q / CB, j = q % CB;
-      if (i > k && j > k && j <= i) t[i][j] -= t[i][k] * t[j][k];
-    }
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < CB * CB; q += blockDim.x) {
-    const int r = q / CB, c = q % CB;
-    if (r < m && c < m) A[(long long)(k0 + r) * nd + k0 + c] = (c <= r) ? t[r][c] : 0.0;
-  }
-}
-
-// Tile row I = K+1+blockIdx.x: X L_KK^T = A_IK  (X overwrites A_IK)
-__global__ void __launch_bounds__(CB * CB / 4) k_chol_panel(double* A, int nd, int K) {
-  EDGE_PDL_ENTRY();
-  __shared__ double L[CB][CB + 1];
-  __shared__ double X[CB][CB + 1];
-  const int k0 = K * CB;
-  const int i0 = (K + 1 + blockIdx.x) * CB;
-  const int mk = min(CB, nd - k0), mi = min(CB, nd - i0);
-  for (int q = threadIdx.x; q < CB * CB; q += blockDim.x) {
-    const int r = q / CB, c = q % CB;
-    L[r][c] = (r < mk && c < mk) ? A[(long long)(k0 + r) * nd + k0 + c] : (r == c ? 1.0 : 0.0);
-    X[r][c] = (r < mi && c < mk) ? A[(long long)(i0 + r) * nd + k0 + c] : 0.0;
-  }
-  __syncthreads();
-  // row r of X: x_r[c] = (a_r[c] - sum_{j<c} x_r[j] L[c][j]) / L[c][c], one thread per row
-  for (int r = threadIdx.x; r < CB; r += blockDim.x) {
-    for (int c = 0; c < CB; ++c) {
-      double v = X[r][c];
-      for (int j = 0; j < c; ++j) v -= X[r][j] * L[c][j];
-      X[r][c] = v / L[c][c];
-    }
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < CB * CB; q += blockDim.x) {
-    const int r = q / CB, c = q % CB;
-    if (r < mi && c < mk) A[(long long)(i0 + r) * nd + k0 + c] = X[r][c];
-  }
-}
-
-// Trailing update A_IJ -= A_IK A_JK^T for K < J <= I; blockIdx.x enumerates (I, J).
-__global__ void __launch_bounds__(CB * CB / 4) k_chol_update(double* A, int nd, int K, int nt) {
-  EDGE_PDL_ENTRY();
-  __shared__ double P[CB][CB + 1];
-  __shared__ double Q[CB][CB + 1];
-  const int m = nt - K - 1;  // tiles below K
-  int q = blockIdx.x, I = 0;
-  while (q >= I + 1) {  // triangular enumeration: (I, J) with 0 <= J <= I < m
-    q -= I + 1;
-    ++I;
-  }
-  const int J = q;
-  if (I >= m) return;
-  const int k0 = K * CB, i0 = (K + 1 + I) * CB, j0 = (K + 1 + J) * CB;
-  const int mk = min(CB, nd - k0), mi = min(CB, nd - i0), mj = min(CB, nd - j0);
-  for (int t = threadIdx.x; t < CB * CB; t += blockDim.x) {
-    const int r = t / CB, c = t % CB;
-    P[r][c] = (r < mi && c < mk) ? A[(long long)(i0 + r) * nd + k0 + c] : 0.0;
-    Q[r][c] = (r < mj && c < mk) ? A[(long long)(j0 + r) * nd + k0 + c] : 0.0;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < CB * CB; t += blockDim.x) {
-    const int r = t / CB, c = t % CB;
-    if (r >= mi || c >= mj) continue;
-    if (I == J && c > r) continue;
-    double v = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < CB; ++k) v += P[r][k] * Q[c][k];
-    A[(long long)(i0 + r) * nd + j0 + c] -= v;
-  }
-}
-
-// U = L^T (row-major), so that both substitutions below read rows.
-__global__ void k_transpose_lower(const double* __restrict__ L, double* __restrict__ U, int nd) {
-  EDGE_PDL_ENTRY();
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q >= (long long)nd * nd) return;
-  const int r = (int)(q / nd), c = (int)(q % nd);
-  U[(long long)c * nd + r] = (c <= r) ? L[q] : 0.0;
-}
-
-// Column `col` of A^-1 = L^-T L^-1 e_col, one block per column.  U = L^T row-major.
-__global__ void __launch_bounds__(256) k_chol_inverse(const double* __restrict__ L, const double* __restrict__ U,
-                                                      double* __restrict__ X, int nd) {
-  EDGE_PDL_ENTRY();
-  extern __shared__ double y[];
-  const int col = blockIdx.x;
-  const int t = threadIdx.x, nt = blockDim.x;
-  for (int i = t; i < nd; i += nt) y[i] = (i == col) ? 1.0 : 0.0;
-  __syncthreads();
-  for (int k = col; k < nd; ++k) {  // L y = e_col (y_i = 0 for i < col)
-    const double yk = y[k] / U[(long long)k * nd + k];
-    __syncthreads();
-    if (t == 0) y[k] = yk;
-    for (int i = k + 1 + t; i < nd; i += nt) y[i] -= U[(long long)k * nd + i] * yk;
-    __syncthreads();
-  }
-  for (int k = nd - 1; k >= 0; --k) {  // L^T x = y
-    const double xk = y[k] / L[(long long)k * nd + k];
-    __syncthreads();
-    if (t == 0) y[k] = xk;
-    for (int i = t; i < k; i += nt) y[i] -= L[(long long)k * nd + i] * xk;
-    __syncthreads();
-  }
-  for (int i = t; i < nd; i += nt) X[(long long)i * nd + col] = y[i];
-}
-
 // x = Ainv b on the coarsest level: b and x in slot layout (types TB/TX), Ainv dense FP64.
 // Each block first gathers b into shared memory in dense order (nd * sizeof(TB) bytes of
 // dynamic shared memory), then one warp per dense row.

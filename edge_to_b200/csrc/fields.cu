@@ -1298,4 +1298,264 @@ int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, cons
   return user3_launch<false>(g, K, nullptr, nullptr, nullptr, 0, u, dk, stream);
 }
 
+// ------------------------------------------------------------------ coarsest level
+// Inverse of the coarsest Galerkin matrix by the symmetric sweep (Gauss-Jordan) on 64 x 64 blocks: for
+// every block column K, with P = A_KK^-1,
+//   A_KK <- -P,   A_iK <- A_iK P,   A_ij <- A_ij - A_iK P A_Kj   (i, j != K),
+// after all of which A holds -A^-1; a positive definite matrix needs no pivoting (its pivots are the
+// squares of the Cholesky diagonal, checked as they come).  Only the blocks on and below the diagonal
+// are kept.  Per K two launches: the panel A_iK P, and the rank-64 update of all other blocks, whose
+// block (K + 1, K + 1) goes on to invert itself so that the next panel can start.  Every product is a
+// 64 x 64 x 64 FP64 tile product (4 x 4 outputs per thread, operands k-major in shared memory).
+//
+// What bounds it: the nt = nd / 64 steps in sequence for small matrices (a block's own inverse is a
+// chain of 64 sweeps, 24 us), FP64 rate (nd^3 operations) and the tiles' way through L2 for large ones:
+// 0.13 ms at nd = 135 and 192, 0.46 at 675, 2.1 at 2,352, 7.3 at 4,131.  The blocked Cholesky
+// factorisation with one block per column of the inverse that it replaces was a chain of 2 nd
+// barrier-separated vector updates on a factor reread by every column: 13 ms at 2,352, 110 at 4,131.
+constexpr int INV_T = 256;
+
+// acc -= L R^T for k-major operands L[k][r], R[k][c], k < KD, with rows of LD doubles in shared memory
+template <int KD, int LD, bool MINUS> EDGE_D void tile_mac(const double* L, const double* R, double acc[4][4]) {
+  L += (threadIdx.x >> 4) * 4;
+  R += (threadIdx.x & 15) * 4;
+#pragma unroll 4
+  for (int k = 0; k < KD; ++k, L += LD, R += LD) {
+    double a[4], b[4];
+    *reinterpret_cast<double2*>(a) = *reinterpret_cast<const double2*>(L);
+    *reinterpret_cast<double2*>(a + 2) = *reinterpret_cast<const double2*>(L + 2);
+    *reinterpret_cast<double2*>(b) = *reinterpret_cast<const double2*>(R);
+    *reinterpret_cast<double2*>(b + 2) = *reinterpret_cast<const double2*>(R + 2);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fma(MINUS ? -a[i] : a[i], b[j], acc[i][j]);
+  }
+}
+
+// P = a^-1 of the block whose 4 x 4 pieces the threads hold: scalar sweeps a_rc <- a_rc - v_r v_c / d
+// with v column k and d = v_k.  The pivot's row and column take the same update from zero with
+// -1 / d in place of v_r / d and -1 in place of v_c.  One barrier per sweep: the owners of the next
+// pivot's column publish it as soon as they have updated it.  sv: 2 x 64 doubles.
+EDGE_D void block_invert(double a[4][4], double* sv, double* __restrict__ P, int* status) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  if (tx == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sv[ty * 4 + i] = a[i][0];
+  }
+  __syncthreads();
+  bool bad = false;
+  for (int kb = 0; kb < 16; ++kb) {
+    const bool mr = ty == kb, mc = tx == kb;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int k = kb * 4 + kk;
+      const double* v = sv + (k & 1) * INV_B;
+      double d = v[k];
+      double vr[4], vc[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        vr[i] = v[ty * 4 + i];
+        vc[i] = v[tx * 4 + i];
+      }
+      if (!(d > 0.0)) {
+        bad = true;
+        d = 1.0;
+      }
+      const double inv = 1.0 / d;
+      if (mr) vr[kk] = -1.0;
+      if (mc) vc[kk] = -1.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) vr[i] *= inv;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (mr) a[kk][i] = 0.0;
+        if (mc) a[i][kk] = 0.0;
+      }
+      // the next pivot's column first
+      const int kn = k + 1;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i][(kk + 1) & 3] = fma(-vr[i], vc[(kk + 1) & 3], a[i][(kk + 1) & 3]);
+      if (kn < INV_B && tx == kn >> 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sv[(kn & 1) * INV_B + ty * 4 + i] = a[i][(kk + 1) & 3];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j != ((kk + 1) & 3))
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i][j] = fma(-vr[i], vc[j], a[i][j]);
+      __syncthreads();
+    }
+  }
+  if (bad && threadIdx.x == 0) *status = 1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) P[(ty * 4 + i) * INV_B + tx * 4 + j] = -a[i][j];
+}
+
+// Unit diagonal on the padding, and the inverse of block (0, 0).
+__global__ void __launch_bounds__(INV_T) k_inv_start(double* __restrict__ A, int nd, int np, double* __restrict__ P, int* status) {
+  EDGE_PDL_ENTRY();
+  __shared__ double sv[2 * INV_B];
+  const int r0 = (threadIdx.x >> 4) * 4, c0 = (threadIdx.x & 15) * 4;
+  for (int i = nd + threadIdx.x; i < np; i += INV_T) A[(long long)i * np + i] = 1.0;
+  __syncthreads();
+  double a[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[i][j] = A[(long long)(r0 + i) * np + c0 + j];
+  block_invert(a, sv, P, status);
+}
+
+// Block i of the panel: R_i = A_iK kept k-major in Rt, W_i = R_i P k-major in Wt and in A.  Shared rows
+// of 66 doubles: the transposed fill meets two-way bank conflicts only.
+constexpr int INV_LD = INV_B + 2;
+__global__ void __launch_bounds__(INV_T)
+k_inv_panel(double* __restrict__ A, int np, int K, const double* __restrict__ P, double* __restrict__ Rt, double* __restrict__ Wt) {
+  EDGE_PDL_ENTRY();
+  extern __shared__ __align__(16) double inv_smem[];
+  double *sR = inv_smem, *sP = sR + INV_B * INV_LD;
+  const int I = blockIdx.x, r0 = (threadIdx.x >> 4) * 4, c0 = (threadIdx.x & 15) * 4;
+  const long long iB = (long long)I * INV_B, kB = (long long)K * INV_B;
+  if (I == K) {
+    for (int q = threadIdx.x; q < INV_B * INV_B; q += INV_T)
+      A[(kB + q / INV_B) * np + kB + q % INV_B] = -P[q];
+    return;
+  }
+#pragma unroll
+  for (int t = 0; t < INV_B * INV_B / INV_T; ++t) {
+    const int q = threadIdx.x + t * INV_T, x = q / INV_B, y = q % INV_B;
+    sP[x * INV_LD + y] = P[q];
+    if (I > K) sR[y * INV_LD + x] = A[(iB + x) * np + kB + y];
+    else sR[x * INV_LD + y] = A[(kB + x) * np + iB + y];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < INV_B * INV_B; q += INV_T)
+    Rt[(q / INV_B) * (long long)np + iB + q % INV_B] = sR[q / INV_B * INV_LD + q % INV_B];
+  double acc[4][4] = {};
+  tile_mac<INV_B, INV_LD, false>(sR, sP, acc);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sR[(c0 + j) * INV_LD + r0 + i] = acc[i][j];
+      if (I > K) A[(iB + r0 + i) * np + kB + c0 + j] = acc[i][j];
+    }
+  __syncthreads();
+  for (int q = threadIdx.x; q < INV_B * INV_B; q += INV_T) {
+    const int k = q / INV_B, r = q % INV_B;
+    const double v = sR[k * INV_LD + r];
+    Wt[k * (long long)np + iB + r] = v;
+    if (I < K) A[(kB + k) * np + iB + r] = v;
+  }
+}
+
+EDGE_D void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// A_ij -= W_i R_j^T for the blocks i >= j other than row and column K.  All of a tile's operands are
+// requested at once (the second half of the depth arrives while the first is multiplied).  The block
+// that inverts itself at the end is the first of the grid, so that this overlaps the other tiles.
+__global__ void __launch_bounds__(INV_T, 3)
+k_inv_update(double* __restrict__ A, int np, int K, const double* __restrict__ Rt, const double* __restrict__ Wt,
+             double* __restrict__ Pnext, int* status) {
+  EDGE_PDL_ENTRY();
+  extern __shared__ __align__(16) double inv_smem[];
+  double *sW = inv_smem, *sR = sW + INV_B * INV_B;
+  int q = blockIdx.x;
+  const int qd = (K + 1) * (K + 2) / 2 + K + 1;  // block (K + 1, K + 1)
+  if (qd < (int)gridDim.x) q = q == 0 ? qd : q == qd ? 0 : q;
+  int I = (int)((sqrtf(8.f * q + 1.f) - 1.f) * 0.5f);
+  while ((I + 1) * (I + 2) / 2 <= q) ++I;
+  while (I * (I + 1) / 2 > q) --I;
+  const int J = q - I * (I + 1) / 2;
+  if (I == K || J == K) return;
+  const long long iB = (long long)I * INV_B, jB = (long long)J * INV_B;
+  const int r0 = (threadIdx.x >> 4) * 4, c0 = (threadIdx.x & 15) * 4;
+  constexpr int H = INV_B / 2;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int t = 0; t < H * INV_B / 2 / INV_T; ++t) {
+      const int p = threadIdx.x + t * INV_T, k = h * H + p / (INV_B / 2), c = 2 * (p % (INV_B / 2));
+      cp_async16(sW + k * INV_B + c, Wt + (long long)k * np + iB + c);
+      cp_async16(sR + k * INV_B + c, Rt + (long long)k * np + jB + c);
+    }
+    cp_commit();
+  }
+  double a[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; j += 2)
+      *reinterpret_cast<double2*>(&a[i][j]) = *reinterpret_cast<const double2*>(A + (iB + r0 + i) * np + jB + c0 + j);
+  cp_wait<1>();
+  __syncthreads();
+  tile_mac<H, INV_B, true>(sW, sR, a);
+  cp_wait<0>();
+  __syncthreads();
+  tile_mac<H, INV_B, true>(sW + H * INV_B, sR + H * INV_B, a);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; j += 2)
+      *reinterpret_cast<double2*>(A + (iB + r0 + i) * np + jB + c0 + j) = *reinterpret_cast<const double2*>(&a[i][j]);
+  if (I == K + 1 && J == K + 1) {
+    __syncthreads();
+    block_invert(a, sW, Pnext, status);
+  }
+}
+
+__global__ void k_inv_finish(const double* __restrict__ A, int nd, int np, double* __restrict__ Ainv) {
+  EDGE_PDL_ENTRY();
+  __shared__ double t[32][33];
+  // block (by, bx) of 32 x 32 with by >= bx: written in place and mirrored
+  const int bx = blockIdx.x, by = blockIdx.y;
+  if (bx > by) return;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int r = y; r < 32; r += 8) {
+    const int row = by * 32 + r, col = bx * 32 + x;
+    double v = 0.0;
+    if (row < nd && col < nd) v = -A[(long long)(row >= col ? row : col) * np + (row >= col ? col : row)];
+    t[r][x] = v;
+    if (row < nd && col < nd) Ainv[(long long)row * nd + col] = v;
+  }
+  __syncthreads();
+  if (bx == by) return;
+  for (int r = y; r < 32; r += 8) {
+    const int row = bx * 32 + r, col = by * 32 + x;
+    if (row < nd && col < nd) Ainv[(long long)row * nd + col] = t[x][r];
+  }
+}
+
+int spd_inverse(double* A, int nd, double* Ainv, double* work, int* status, cudaStream_t stream) {
+  const int np = inv_padded(nd), nt = np / INV_B;
+  double *Rt = work, *Wt = Rt + (long long)INV_B * np, *P0 = Wt + (long long)INV_B * np, *P1 = P0 + INV_B * INV_B;
+  constexpr int psmem = 2 * INV_B * INV_LD * 8, usmem = 2 * INV_B * INV_B * 8;
+  static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
+  if (!attr.load()) {
+    if (cudaFuncSetAttribute(k_inv_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_inv_update, cudaFuncAttributeMaxDynamicSharedMemorySize, usmem) != cudaSuccess)
+      return 0;
+    attr = true;
+  }
+  k_inv_start<<<1, INV_T, 0, stream>>>(A, nd, np, P0, status);
+  int n = 1;
+  for (int K = 0; K < nt; ++K) {
+    k_inv_panel<<<nt, INV_T, psmem, stream>>>(A, np, K, (K & 1) ? P1 : P0, Rt, Wt);
+    ++n;
+    if (nt > 1) {
+      k_inv_update<<<nt * (nt + 1) / 2, INV_T, usmem, stream>>>(A, np, K, Rt, Wt, (K & 1) ? P0 : P1, status);
+      ++n;
+    }
+  }
+  const unsigned nb = (unsigned)((nd + 31) / 32);
+  k_inv_finish<<<dim3(nb, nb), 256, 0, stream>>>(A, nd, np, Ainv);
+  return n + 1;
+}
+
 }  // namespace edge

@@ -102,4 +102,13 @@ int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, cons
 // Grids that the launches above take (their tile counts are grid dimensions).
 bool user_grid_ok(const Geo& g);
 
+// ------------------------------------------------------------------ coarsest level
+// Inverse of a symmetric positive definite matrix.  A: np x np row-major, np = inv_padded(nd), the nd x nd
+// matrix in its upper left corner and zeros elsewhere (overwritten); Ainv: nd x nd; work: inv_work(nd)
+// doubles.  *status is set to 1 on a pivot that is not positive (taken as 1 then).
+constexpr int INV_B = 64;
+inline int inv_padded(int nd) { return (nd + INV_B - 1) / INV_B * INV_B; }
+inline long long inv_work(int nd) { return 2LL * INV_B * inv_padded(nd) + 2LL * INV_B * INV_B; }
+int spd_inverse(double* A, int nd, double* Ainv, double* work, int* status, cudaStream_t stream);
+
 }  // namespace edge

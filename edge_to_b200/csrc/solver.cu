@@ -305,7 +305,7 @@ struct Prob {
   std::vector<int> w_levels;
   std::vector<Level> lv;
   int nd = 0;
-  double *Adense = nullptr, *Ainv = nullptr, *Ut = nullptr;
+  double *Adense = nullptr, *Ainv = nullptr, *inv_work = nullptr;
   // 3-D Galerkin products of the stencil levels as three one-axis passes (k_galerkin3_axis)
   // through two FP64 intermediates sized for the level 1 -> 2 product; false: k_galerkin3_st
   bool gal_axis = true;
@@ -1124,27 +1124,14 @@ static void mg_setup(Prob& P) {
       }
     }
   }
-  // coarsest: dense FP64 Cholesky and explicit inverse
+  // coarsest: dense FP64 inverse
   const Geo& gL = P.lv[L].g;
   const int nd = P.nd;
-  CK(cudaMemsetAsync(P.Adense, 0, (size_t)nd * nd * sizeof(double), P.stream));
-  launch(P, k_st_to_dense<T>, cdiv(gL.n, 256), 256, 0, gL, (const T*)P.lv[L].S, P.Adense, nd);
-  KCHECK();
+  const int np = inv_padded(nd);
+  CK(cudaMemsetAsync(P.Adense, 0, (size_t)np * np * sizeof(double), P.stream));
+  launch(P, k_st_to_dense<T>, cdiv(gL.n, 256), 256, 0, gL, (const T*)P.lv[L].S, P.Adense, np);
   CK(cudaMemsetAsync(P.chol_status, 0, sizeof(int), P.stream));
-  const int nt = (nd + CB - 1) / CB;
-  for (int K = 0; K < nt; ++K) {
-    launch(P, k_chol_diag, 1, CB * CB / 4, 0, P.Adense, nd, K, P.chol_status);
-    if (K + 1 < nt) {
-      launch(P, k_chol_panel, nt - K - 1, CB * CB / 4, 0, P.Adense, nd, K);
-      const int m = nt - K - 1;
-      launch(P, k_chol_update, m * (m + 1) / 2, CB * CB / 4, 0, P.Adense, nd, K, nt);
-    }
-  }
-  KCHECK();
-  launch(P, k_transpose_lower, cdiv((long long)nd * nd, 256), 256, 0, P.Adense, P.Ut, nd);
-  if (nd * sizeof(double) > 48 * 1024)
-    CK(cudaFuncSetAttribute(k_chol_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nd * sizeof(double))));
-  launch(P, k_chol_inverse, nd, 256, nd * sizeof(double), P.Adense, P.Ut, P.Ainv, nd);
+  P.nlaunch += spd_inverse(P.Adense, nd, P.Ainv, P.inv_work, P.chol_status, P.stream);
   KCHECK();
 }
 
@@ -1432,9 +1419,9 @@ static void mg_allocate(Prob& P) {
     P.tail_bar = P.alloc<unsigned>(2);
     CK(cudaMemset(P.tail_bar, 0, 2 * sizeof(unsigned)));
   }
-  P.Adense = P.alloc<double>((size_t)P.nd * P.nd);
+  P.Adense = P.alloc<double>((size_t)inv_padded(P.nd) * inv_padded(P.nd));
   P.Ainv = P.alloc<double>((size_t)P.nd * P.nd);
-  P.Ut = P.alloc<double>((size_t)P.nd * P.nd);
+  P.inv_work = P.alloc<double>((size_t)inv_work(P.nd));
   if (P.dim == 3 && L >= 2) {  // the largest stencil product, level 1 -> 2
     Geo g1, g2;
     gal_axis_geos(P.lv[1].g, P.lv[2].g, g1, g2);
@@ -2906,7 +2893,7 @@ int edge_mg_config(edge_problem* p, int n_level, int n_smooth, double omega, dou
         }
       }
     }
-    for (void* q : {(void*)P.Adense, (void*)P.Ainv, (void*)P.Ut, (void*)P.gal_t1, (void*)P.gal_t2}) {
+    for (void* q : {(void*)P.Adense, (void*)P.Ainv, (void*)P.inv_work, (void*)P.gal_t1, (void*)P.gal_t2}) {
       if (!q) continue;
       auto it = std::find(P.allocs.begin(), P.allocs.end(), q);
       if (it != P.allocs.end()) {

@@ -4,8 +4,8 @@
 Same constructor keywords and the same algorithm: Galerkin hierarchy rebuilt on every
 solve, damped-Jacobi V-cycle with omega*1.06^level, exact coarsest solve, PCG with warm
 start from the last solution and the residual-driven omega schedule; omega is reset to
-min_omega at the start of each solve as the GPU reference does.  The coarsest level is
-factorised by a dense FP64 Cholesky on the GPU (exact, like the reference's splu), so
+min_omega at the start of each solve as the GPU reference does.  The coarsest matrix is
+inverted in dense FP64 on the GPU (exact, like the reference's splu), so
 coarse_solver only selects between equivalent exact solves.
 """
 import ctypes

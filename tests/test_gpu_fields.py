@@ -5,7 +5,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from oracle import topopt
+from oracle import ops, topopt
 
 pytestmark = pytest.mark.gpu
 
@@ -114,3 +114,26 @@ def test_product_and_energy_on_user_vectors(nel, box):
             np.testing.assert_allclose(k.process_grad(x).cpu().numpy(), dk, rtol=0, atol=1e-13)
         twice, _ = _dense(mesh, nel, E, ref, c)
         np.testing.assert_allclose(k.dot(k.dot(ut)).cpu().numpy(), twice, rtol=0, atol=2e-13)
+
+
+@pytest.mark.parametrize("nel", [(2, 2), (6, 4), (12, 12), (14, 14), (16, 14), (30, 62), (62, 62), (4, 4, 4), (8, 6, 6),
+                                 (10, 8, 8)])
+def test_coarsest_inverse_solves_a_two_level_system(nel):
+    """Coarsest matrices of 8 to 2,048 DOFs (blocks of 64: fewer, exactly one, two, one DOF more, many): the
+    two-level V-cycle's PCG takes the oracle's iterations and reaches its solution, as it only does
+    with the exact coarsest solve (rtol 1e-10; condition numbers below 1e5)."""
+    import torch
+    import edge_to_b200 as eb
+    dim = len(nel)
+    p = (topopt.mbb_problem if dim == 2 else topopt.cantilever_problem)(
+        *nel, vf=0.4, mg_kwargs=dict(tol=1e-10, n_level=1, maxiter=300, variant="gpu"))
+    E = np.random.default_rng(4).uniform(0.3, 1.0, p.grid.n_el) ** 3
+    ref, _ = p.solver.solve(ops.assemble(p.grid, p.K0, E, p.cons), p.f, use_last=False)
+    mesh = (eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D)(
+        *nel, *map(float, nel), stiffness=lambda x: eb.auto_stiffness(x, 1.0, 0.3))
+    k = eb.CuStructuredStiffnessKernel(mesh)
+    k.add_constraints(p.cons)
+    sv = eb.CuMultiGrid(mesh, k, tol=1e-10, n_level=1, maxiter=300)
+    x, res = sv.solve(torch.as_tensor(p.f, device="cuda"), torch.as_tensor(E, device="cuda"), use_last=False)
+    assert res < 1e-10 and sv.last_iters == p.solver.pcg_iters[-1]
+    np.testing.assert_allclose(x.cpu().numpy(), ref, rtol=0, atol=1e-9 * np.abs(ref).max())
