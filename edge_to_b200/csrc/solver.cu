@@ -3660,7 +3660,11 @@ struct edge_batch {
   BatchDesc* h_desc = nullptr;
   double** d_scal = nullptr;
   double** h_scal = nullptr;
+  static constexpr int NQ = 8;  // queue counters: one per launch of a solve
   unsigned* queue = nullptr;
+  // a batch that fits on the GPU at once: the team size of each queue position (sorted, largest first),
+  // one launch per size; empty: teams of `team` blocks and a queue
+  std::vector<int> sized;
   double *d_res = nullptr, *d_comp = nullptr;
   int *d_iters = nullptr, *d_done = nullptr;
   double *h_res = nullptr, *h_comp = nullptr;
@@ -3702,6 +3706,7 @@ template <typename TV, typename TD0, typename TS, int BT, int C>
 static void batch_go(Prob& P0, edge_batch& B, int off, int cnt, int qslot, int sm_budget, cudaStream_t stream,
                      double tol, int maxiter) {
   auto kern = k_batch_pcg<TV, TD0, TS, BT, C>;
+  if constexpr (C > 8) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   int dev = 0, sms = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -3743,6 +3748,7 @@ static void batch_go_team(Prob& P0, edge_batch& B, int team, int off, int cnt, i
     case 2: batch_go<TV, TD0, TS, BT, 2>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
     case 4: batch_go<TV, TD0, TS, BT, 4>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
     case 8: batch_go<TV, TD0, TS, BT, 8>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
+    case 16: batch_go<TV, TD0, TS, BT, 16>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
     default: batch_go<TV, TD0, TS, BT, 1>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
   }
 }
@@ -3756,6 +3762,87 @@ static void batch_group(Prob& P0, edge_batch& B, int threads, int team, int off,
   else
     batch_go_team<TV, TD0, TS, 512>(P0, B, team, off, cnt, qslot, sm_budget, stream, tol, maxiter);
 }
+// Clusters of 16 blocks of the solve kernel that the GPU holds at once (0: none).
+template <typename TV, typename TD0, typename TS, int BT> static int batch_clusters16() {
+  auto kern = k_batch_pcg<TV, TD0, TS, BT, 16>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3(BT);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+
+// Team sizes of a batch whose problems all fit on the GPU at once.  With teams of one size such a batch
+// takes as long as its costliest problem while SMs stay idle (24 problems of 10k-220k DOFs on teams
+// of four: 285 ms, the mean problem 90).  A problem's solve takes about its iterations times
+// (I_c + DOFs / c) on c blocks (fitted to 24 problems at c = 1, 4 and 8: a step of a team costs a
+// barrier and two trips to L2 whatever the size; a single block's barrier is nearly free), so the
+// smallest time T is sought for which the smallest sizes with time <= T fit.  Sizes are powers of two
+// up to 16 and their sum stays within the blocks that clusters of 16 could fill: powers of two then
+// pack into the GPCs.  24 problems: 285 -> 160 ms (every SM busy, problems end between 92 and 160 ms);
+// 8 and 17 problems: calls of 275 and 296 ms take 107 and 119.  Returns the sizes by queue position
+// and the predicted time of that choice.
+static double batch_sizes(const edge_batch& B, int budget, std::vector<int>& size) {
+  static const int SZ[5] = {1, 2, 4, 8, 16};
+  const int n = (int)B.order.size();
+  auto time = [&](int k, int c) {
+    const double dof = (double)std::max<long long>(1, B.probs[B.order[k]]->P.n_dof);
+    const double its = std::max(1.0, (double)B.cost[B.order[k]] / dof);
+    return its * ((c == 1 ? 500.0 : 5800.0) + dof / c);
+  };
+  std::vector<double> ts;
+  for (int k = 0; k < n; ++k)
+    for (int c : SZ) ts.push_back(time(k, c));
+  std::sort(ts.begin(), ts.end());
+  auto fits = [&](double T, std::vector<int>* out) {
+    long long sum = 0;
+    for (int k = 0; k < n; ++k) {
+      int c = 0;
+      for (int t : SZ)
+        if (time(k, t) <= T) {
+          c = t;
+          break;
+        }
+      if (!c) return false;
+      if (out) (*out)[k] = c;
+      sum += c;
+    }
+    return sum <= budget;
+  };
+  size_t lo = 0, hi = ts.size();
+  while (lo < hi) {  // the smallest T that fits
+    const size_t mid = (lo + hi) / 2;
+    if (fits(ts[mid], nullptr)) hi = mid;
+    else lo = mid + 1;
+  }
+  if (lo == ts.size()) return -1.0;
+  size.assign(n, 0);
+  fits(ts[lo], &size);
+  return ts[lo];
+}
+// The time of the same batch from the queue on teams of `team` blocks.
+static double batch_queue_time(const edge_batch& B, int sms) {
+  double most = 0.0, sum = 0.0;
+  for (int i : B.order) {
+    const double dof = (double)std::max<long long>(1, B.probs[i]->P.n_dof);
+    const double t = std::max(1.0, (double)B.cost[i] / dof) * ((B.team == 1 ? 500.0 : 5800.0) + dof / B.team);
+    most = std::max(most, t);
+    sum += t;
+  }
+  return std::max(most, sum / std::max(1, sms / B.team));
+}
+
 // The solve launch(es): problems below B.split_dof DOFs (when a team of several blocks is
 // configured) are solved by single blocks in a second launch beside the teams' launch, on its
 // own share of the SMs (proportional to the groups' expected work), since a team's barriers
@@ -3763,6 +3850,23 @@ static void batch_group(Prob& P0, edge_batch& B, int threads, int team, int off,
 template <typename TV, typename TD0, typename TS>
 static void batch_launch(Prob& P0, edge_batch& B, int n, int n_large, double w_large, double w_small,
                          cudaStream_t s, double tol, int maxiter) {
+  if (!B.sized.empty()) {  // one launch per team size, side by side
+    CK(cudaEventRecord(B.fork, s));
+    int g = 0;
+    for (int k = 0; k < n; ++g) {
+      int e = k;
+      while (e < n && B.sized[e] == B.sized[k]) ++e;
+      cudaStream_t st = g == 0 ? s : B.side[g];
+      if (g) CK(cudaStreamWaitEvent(st, B.fork, 0));
+      batch_group<TV, TD0, TS>(P0, B, B.threads, B.sized[k], k, e - k, g, 0, st, tol, maxiter);
+      k = e;
+    }
+    for (int q = 1; q < g; ++q) {
+      CK(cudaEventRecord(B.join[q], B.side[q]));
+      CK(cudaStreamWaitEvent(s, B.join[q], 0));
+    }
+    return;
+  }
   if (B.team == 1 || n_large == n || n_large == 0) {
     batch_group<TV, TD0, TS>(P0, B, B.threads, B.team, 0, n, 0, 0, s, tol, maxiter);
     return;
@@ -3813,7 +3917,7 @@ int edge_batch_create(int n, edge_problem* const* problems, edge_filter* const* 
   CK(cudaMallocHost(&B->h_desc, n * sizeof(BatchDesc)));
   CK(cudaMalloc(&B->d_scal, n * sizeof(double*)));
   CK(cudaMallocHost(&B->h_scal, n * sizeof(double*)));
-  CK(cudaMalloc(&B->queue, 2 * sizeof(unsigned)));
+  CK(cudaMalloc(&B->queue, edge_batch::NQ * sizeof(unsigned)));
   CK(cudaMalloc(&B->d_res, n * sizeof(double)));
   CK(cudaMalloc(&B->d_comp, n * sizeof(double)));
   CK(cudaMalloc(&B->d_iters, n * sizeof(int)));
@@ -3966,6 +4070,33 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
   // steps) x the previous PCG iterations
   int n_large = n;
   double w_large = 0.0, w_small = 0.0;
+  B.sized.clear();
+  if (B.team > 1 && B.split_dof == 0 && n <= 148) {
+    int clusters = 0, dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (!mixed)
+      clusters = B.threads == 1024 ? batch_clusters16<double, double, double, 1024>()
+                                   : batch_clusters16<double, double, double, 512>();
+    else if (bf16)
+      clusters = B.threads == 1024 ? batch_clusters16<float, __nv_bfloat16, __nv_bfloat16, 1024>()
+                                   : batch_clusters16<float, __nv_bfloat16, __nv_bfloat16, 512>();
+    else
+      clusters = B.threads == 1024 ? batch_clusters16<float, __nv_bfloat16, float, 1024>()
+                                   : batch_clusters16<float, __nv_bfloat16, float, 512>();
+    std::vector<int> size;
+    const double t = batch_sizes(B, std::min(16 * clusters, sms), size);
+    if (t > 0.0 && t < batch_queue_time(B, sms)) {  // queue positions by size, then by cost
+      std::vector<int> at(n), order(n);
+      for (int k = 0; k < n; ++k) at[k] = k;
+      std::stable_sort(at.begin(), at.end(), [&](int a, int c) { return size[a] > size[c]; });
+      for (int k = 0; k < n; ++k) {
+        order[k] = B.order[at[k]];
+        B.sized.push_back(size[at[k]]);
+      }
+      B.order = order;
+    }
+  }
   if (B.team > 1 && B.split_dof > 0) {
     auto big = [&](int i) { return B.probs[i]->P.n_dof >= B.split_dof; };
     std::stable_partition(B.order.begin(), B.order.end(), big);
@@ -4068,7 +4199,7 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
   try {
     CK(cudaMemcpyAsync(B.d_desc, B.h_desc, n * sizeof(BatchDesc), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(B.d_scal, B.h_scal, n * sizeof(double*), cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(B.queue, 0, 2 * sizeof(unsigned), s));
+    CK(cudaMemsetAsync(B.queue, 0, edge_batch::NQ * sizeof(unsigned), s));
     CK(cudaEventRecord(B.ev[1], s));
     if (!mixed)
       batch_launch<double, double, double>(P0, B, n, n_large, w_large, w_small, s, tol, maxiter);

@@ -353,7 +353,9 @@ int edge_batch_create(int n, edge_problem* const* problems, edge_filter* const* 
 int edge_batch_destroy(edge_batch* b);
 /* Shape of the solve launch: `threads` per block and `team` blocks per problem (team > 1: a
  * thread block cluster of that many blocks solves each problem together).  Supported: team 1
- * with 256, 512 (default) or 1024 threads; team 2, 4 or 8 with 512 or 1024 threads. */
+ * with 256, 512 (default) or 1024 threads; team 2, 4 or 8 with 512 or 1024 threads.  With team > 1,
+ * a batch small enough for all its solves to run at once gets a team size per problem instead (1 to
+ * 16 blocks by its DOFs and previous iterations) when that is predicted to finish sooner. */
 int edge_batch_set_threads(edge_batch* b, int threads, int team);
 /* With team > 1: problems with fewer than split_dof DOFs (default 0 = none) are solved
  * by single blocks of small_threads threads (256, 512 or 1024, the default) in a second
