@@ -31,7 +31,11 @@
 namespace edge {
 
 // The blocks that solve one problem together.  sum(): the team-wide FP64 sum of a per-thread
-// value in a fixed order, returned to every thread; `sh` holds 33 + C doubles of shared memory.
+// value in a fixed order, returned to every thread, and a team barrier; `sh` holds 33 + 2 C doubles of
+// shared memory, `ph` alternates between its two halves from sum to sum (alike in every thread).
+// Each block writes its sum into every block's shared memory, so that after one cluster barrier all
+// threads read locally; all threads reading rank 0's C values through distributed shared memory
+// queued up there, and took a second barrier.
 template <int C> struct Team {
   static EDGE_D unsigned rank() {
     if constexpr (C == 1) return 0;
@@ -43,24 +47,22 @@ template <int C> struct Team {
     if constexpr (C == 1) __syncthreads();
     else cooperative_groups::this_cluster().sync();
   }
-  static EDGE_D double sum(double v, double* sh) {
-    double r = block_sum(v, sh);  // valid in thread 0 of each block
+  static EDGE_D double sum(double v, double* sh, int& ph) {
+    double r = block_sum(v, sh);  // valid in every lane of warp 0 of each block
     if constexpr (C == 1) {
-      __syncthreads();
       if (threadIdx.x == 0) sh[32] = r;
       __syncthreads();
       r = sh[32];
-      __syncthreads();
-      return r;
+      return r;  // sh is written again only behind block_sum's barrier
     } else {
       auto cl = cooperative_groups::this_cluster();
-      if (threadIdx.x == 0) cl.map_shared_rank(sh + 33, 0)[rank()] = r;
+      double* half = sh + 33 + ph * C;
+      if (threadIdx.x < C) *cl.map_shared_rank(half + rank(), threadIdx.x) = r;
       cl.sync();
-      const double* src = cl.map_shared_rank(sh + 33, 0);
       double t = 0.0;
 #pragma unroll
-      for (int k = 0; k < C; ++k) t += src[k];
-      cl.sync();  // rank 0's slots and every block's sh are reused by the next sum
+      for (int k = 0; k < C; ++k) t += half[k];
+      ph ^= 1;  // this half is written again two sums from now, behind the next sum's barrier
       return t;
     }
   }
@@ -88,6 +90,8 @@ struct BatchDesc {
   const void* ET;     // fine-level E in the V-cycle's type
   const double* K0_64;  // element matrix, corner-bit order, FP64
   const void* K0_T;     // the same in the V-cycle's type
+  int wht;              // the element matrix has the box structure: k2 holds its transform
+  KHat2<double> k2;
   double *b64, *x64, *r64, *p64, *q64;
   const double* Ainv;
   PcgState* st;
@@ -103,14 +107,12 @@ struct BatchDesc {
 // node is unconditional (a neighbour or element outside the grid reads the node's own slot
 // and is replaced by zero), so a thread's loads are in flight together: each pass is a few
 // round trips to L2 per node, not one per neighbour.
-// Input of the fine operator: u itself (ArrIn) or a value computed from other arrays
-// (uin(slot, component)).
-template <typename T> struct ArrIn {
-  const T* u;
-  long long n;
-  EDGE_D T operator()(long long ss, int c) const { return u[c * n + ss]; }
-};
-
+// uin(slot, component): the input's values.  The form of the FP64 product, and of any element matrix
+// without the box structure.  The product keeps it where the preconditioner marches in the transform
+// domain (below): on slender problems the solution follows the last bits of the Krylov operator (in 8
+// problems drawn at random the designs moved by 5e-9 of their size with the transform, by 5e-12 with this
+// form), and marching with the full matrix in this order of sums spills at 1024 threads (354 ms a solve of
+// those 8 problems, 171 with this form).
 template <int C, typename T, typename TE, class UIn, class F>
 EDGE_D void b_fine2(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, const T* sK, F&& epi) {
   const int nn = g.nx * g.ny;
@@ -161,6 +163,155 @@ EDGE_D void b_fine2(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, con
   }
 }
 
+// The same operator marching along y, for element matrices with the box structure: a warp owns 32 element
+// columns (30 nodes besides its halo lanes) and a strip of rows, a lane one element per row.  A row
+// costs a lane one node (value, mask) and one E; its right neighbour's node and its left neighbour's
+// contributions come by shuffle, the lower row of nodes and the contributions to the upper one stay in
+// registers, and the element works in the transform domain (10 coefficients, 48 operations) where
+// the node-wise form loads nine nodes and four E and multiplies four 8 x 2 blocks.  The next row's
+// loads are issued a row ahead.  A sweep's pass takes
+// about two thirds of the node-wise pass's time.
+// uin(i, j, s, v): the input at node (i, j), slot s.
+template <int C, typename T, typename TE, class UIn, class F>
+EDGE_D void b_fine2_march(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, const KHat2<T>& K, F&& epi) {
+  const int lane = threadIdx.x & 31, wid = Team<C>::first() >> 5, nwarp = Team<C>::stride() >> 5;
+  const int ct = (g.nx + 29) / 30;                         // column tiles of 30 nodes
+  const int want = nwarp / ct > 0 ? nwarp / ct : 1;        // strips per column tile
+  const int rows = (g.ny + want - 1) / want, strips = (g.ny + rows - 1) / rows;
+  const T k10 = K.dg[0][1], k20 = K.dg[0][2], k30 = K.dg[0][3], k11 = K.dg[1][1], k21 = K.dg[1][2], k31 = K.dg[1][3];
+  const T o01 = K.of[0][1][1], o02 = K.of[0][1][2], o11 = K.of[1][0][1], o12 = K.of[1][0][2];
+  for (int t = wid; t < ct * strips; t += nwarp) {
+    const int cx = t % ct, y0 = (t / ct) * rows, y1 = min(y0 + rows, g.ny);
+    const int i = cx * 30 - 1 + lane;  // this lane's node and element column
+    const bool ni = i >= 0 && i < g.nx;
+    const int ic = ni ? i : 0;
+    struct Row {
+      T raw[2], E;
+      unsigned m;
+    };
+    auto fetch = [&](int j) {  // node (i, j) and the E of element (i, j); clamped loads, zeroed after
+      Row r;
+      const int jc = min(max(j, 0), g.ny - 1);
+      const long long s = g.slot2(ic, jc);
+      const bool in = ni && j >= 0 && j < g.ny;
+      uin(ic, jc, s, r.raw);
+      const unsigned m = __ldg(mask + s);
+      const T e = Conv<T>::from(__ldg(E + s));
+      r.m = in ? m : 3u;
+      r.E = in ? e : T(0);  // slots past the last element hold zero
+      return r;
+    };
+    Row lo = fetch(y0 - 1), hi = fetch(y0);
+    T ul[2], cl[2] = {T(0), T(0)}, cr[2] = {T(0), T(0)};  // masked lower node; contributions carried upwards
+    T ulr[2];                                              // the right neighbour's lower node
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      ul[c] = ((lo.m >> c) & 1) ? T(0) : lo.raw[c];
+      ulr[c] = __shfl_down_sync(0xffffffffu, ul[c], 1);
+    }
+    for (int j = y0 - 1; j < y1; ++j) {  // element row j: nodes j (lo) and j + 1 (hi)
+      const Row nx = fetch(j + 2);
+      T uh[2], uhr[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uh[c] = ((hi.m >> c) & 1) ? T(0) : hi.raw[c];
+        uhr[c] = __shfl_down_sync(0xffffffffu, uh[c], 1);
+      }
+      // transform of the corners b = bx + 2 by, h = hx + 2 hy
+      T q[2][4], v[2][4];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const T sl = ul[c] + ulr[c], dl = ul[c] - ulr[c], su = uh[c] + uhr[c], du = uh[c] - uhr[c];
+        q[c][1] = (dl + du) * lo.E;
+        q[c][2] = (sl - su) * lo.E;
+        q[c][3] = (dl - du) * lo.E;
+      }
+      v[0][1] = k10 * q[0][1] + o01 * q[1][2];
+      v[0][2] = k20 * q[0][2] + o02 * q[1][1];
+      v[0][3] = k30 * q[0][3];
+      v[1][1] = k11 * q[1][1] + o11 * q[0][2];
+      v[1][2] = k21 * q[1][2] + o12 * q[0][1];
+      v[1][3] = k31 * q[1][3];
+      T Au[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        // contributions to corners (0,0) (1,0) (0,1) (1,1); h = 0 vanishes
+        const T a = v[c][1] + v[c][2], b = v[c][2] - v[c][1], d = v[c][1] - v[c][2];
+        const T f00 = a + v[c][3], f10 = b - v[c][3], f01 = d - v[c][3], f11 = v[c][3] - a;
+        // node (i, j): this element's corner (0,0), the left element's (1,0), and the row below's
+        // (0,1) and (1,1) carried from the previous row
+        Au[c] = f00 + cl[c] + __shfl_up_sync(0xffffffffu, f10 + cr[c], 1);
+        cl[c] = f01;
+        cr[c] = f11;
+      }
+      if (j >= y0 && lane >= 1 && lane <= 30 && ni) {
+        const long long s = g.slot2(i, j);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          if ((lo.m >> c) & 1) Au[c] = lo.raw[c];
+        epi(s, lo.raw, Au);
+      }
+      lo = hi;
+      hi = nx;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        ul[c] = uh[c];
+        ulr[c] = uhr[c];
+      }
+    }
+  }
+}
+// The element matrix of a problem in shared memory: dense, and its transform when it has the box
+// structure (else null).
+template <typename T> struct FineK {
+  const T* dense;
+  const KHat2<T>* k2;
+};
+// Input values of the fine operator: an array of the level.
+template <typename T> struct NodeIn {
+  const T* u;
+  long long n;
+  EDGE_D void operator()(int, int, long long s, T v[2]) const {
+    v[0] = u[s];
+    v[1] = u[n + s];
+  }
+};
+// ... or the interpolation of a coarse array (b_prolong2's values: the mean over a node's parents; an
+// even coordinate counts its one parent twice).
+template <typename T> struct ProlongIn {
+  Geo gc;
+  const T* e;
+  EDGE_D void operator()(int i, int j, long long, T v[2]) const {
+    v[0] = v[1] = T(0);
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int ci = min((i + a) >> 1, gc.nx - 1), cj = min((j + b) >> 1, gc.ny - 1);
+        const T iw = inv_bnd_total2<T>(is_bnd(ci, gc.nx) + is_bnd(cj, gc.ny));
+        const long long sc = gc.slot2(ci, cj);
+        v[0] += e[sc] * iw;
+        v[1] += e[gc.n + sc] * iw;
+      }
+    v[0] *= T(0.25);
+    v[1] *= T(0.25);
+  }
+};
+// The fine-level operator in either form; uin(i, j, s, v) as above.
+template <int C, typename T, typename TE, class UIn, class F>
+EDGE_D void b_fine2_op(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, const FineK<T>& K, F&& epi) {
+  if (K.k2) {
+    b_fine2_march<C, T, TE>(g, uin, E, mask, *K.k2, epi);
+  } else {
+    const T* sK = K.dense;
+    b_fine2<C, T, TE>(g, [&](long long ss, int c) {
+      T v[2];
+      uin((int)(ss % g.pz), (int)(ss / g.pz), ss, v);
+      return v[c];
+    }, E, mask, sK, epi);
+  }
+}
+
 // Symmetric 2-D stencil (levels >= 1), one pass of the block over the level's nodes, the
 // sums of k_st2_apply in its order (a neighbour outside the grid reads the node's own slots
 // and contributes zero, so no load is conditional).
@@ -202,27 +353,38 @@ EDGE_D void b_st2(const Geo& g, const T* u, const TS* S, F&& epi) {
   }
 }
 
-// Full-weighting restriction to the coarse nodes (k_restrict2's sums).
+// Full-weighting restriction to the coarse nodes (k_restrict2's sums); with x given, also the coarse
+// level's first sweep from zero, x = w Dinv out.
 template <int C, typename T>
-EDGE_D void b_restrict2(const Geo& gf, const Geo& gc, const T* in, T* out) {
+EDGE_D void b_restrict2(const Geo& gf, const Geo& gc, const T* in, T* out, const T* dinv, T w, T* x) {
   const int nc = gc.nx * gc.ny;
   for (int t = Team<C>::first(); t < nc; t += Team<C>::stride()) {
     const int I = t % gc.nx, J = t / gc.nx;
     const T iw = inv_bnd_total2<T>(is_bnd(I, gc.nx) + is_bnd(J, gc.ny));
     T v[2] = {0, 0};
+#pragma unroll
     for (int di = -1; di <= 1; ++di) {
       const int fi = 2 * I + di;
-      if (fi < 0 || fi >= gf.nx) continue;
-      for (int dj = -1; dj <= 1; ++dj) {
+#pragma unroll
+      for (int dj = -1; dj <= 1; ++dj) {  // unconditional loads: outside the grid the centre, weight 0
         const int fj = 2 * J + dj;
-        if (fj < 0 || fj >= gf.ny) continue;
-        const T w = (T)dist_w(abs(di) + abs(dj));
-        const long long sf = gf.slot2(fi, fj);
-        for (int c = 0; c < 2; ++c) v[c] += w * in[c * gf.n + sf];
+        const bool ok = fi >= 0 && fi < gf.nx && fj >= 0 && fj < gf.ny;
+        const T wt = ok ? (T)(0.25 * (2 - (di != 0)) * (2 - (dj != 0))) : T(0);
+        const long long sf = gf.slot2(ok ? fi : 2 * I, ok ? fj : 2 * J);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const T a = in[c * gf.n + sf];
+          v[c] += ok ? wt * a : T(0);
+        }
       }
     }
     const long long sc = gc.slot2(I, J);
-    for (int c = 0; c < 2; ++c) out[c * gc.n + sc] = v[c] * iw;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const T o = v[c] * iw;
+      out[c * gc.n + sc] = o;
+      if (x) x[c * gc.n + sc] = w * __ldg(dinv + c * gc.n + sc) * o;
+    }
   }
 }
 
@@ -274,18 +436,18 @@ EDGE_D void b_coarse2(const Geo& g, const double* Ainv, int nd, const T* b, T* x
 }
 
 template <int C, typename TA, typename TB>
-EDGE_D double b_dot(long long nv, const TA* a, const TB* b, double* sh) {
+EDGE_D double b_dot(long long nv, const TA* a, const TB* b, double* sh, int& ph) {
   double acc = 0.0;
   for (long long q = Team<C>::first(); q < nv; q += Team<C>::stride()) acc += (double)a[q] * (double)b[q];
-  return Team<C>::sum(acc, sh);
+  return Team<C>::sum(acc, sh, ph);
 }
 
 // One application of level l's operator (fine: the element operator in TV; coarser: the
 // stencil in TS, arithmetic in TV).
 template <int C, typename TV, typename TS, class F>
-EDGE_D void b_level_op(const BatchDesc& d, int l, const TV* u, const TV* sK, F&& epi) {
+EDGE_D void b_level_op(const BatchDesc& d, int l, const TV* u, const FineK<TV>& sK, F&& epi) {
   if (l == 0)
-    b_fine2<C, TV, TV>(d.lv[0].g, ArrIn<TV>{u, d.lv[0].g.n}, (const TV*)d.ET, d.mask, sK, epi);
+    b_fine2_op<C, TV, TV>(d.lv[0].g, NodeIn<TV>{u, d.lv[0].g.n}, (const TV*)d.ET, d.mask, sK, epi);
   else
     b_st2<C, TV, TS>(d.lv[l].g, u, (const TS*)d.lv[l].S, epi);
 }
@@ -298,9 +460,9 @@ EDGE_D void b_level_op(const BatchDesc& d, int l, const TV* u, const TV* sK, F&&
 // out = xb + (e + w Dinv (r - A e)) with xb the down pass's x (recomputed as w Dinv b when
 // fused0); with dot, acc += dotv . out (the PCG's r.z) per thread.
 template <int C, typename TV, typename TS, typename TD, typename TB>
-EDGE_D void b_smooth_level(const BatchDesc& d, int l, const TV* sK, TV w, const TB* b, const TV* xb, TV*& x, TV*& y,
-                           TV*& e1, TV*& e2, TV* r, TV* out, bool down, bool fused0, const double* dotv,
-                           double& acc) {
+EDGE_D void b_smooth_level(const BatchDesc& d, int l, const FineK<TV>& sK, TV w, const TB* b, const TV* xb, TV*& x, TV*& y,
+                           TV*& e1, TV*& e2, TV* r, TV* out, bool down, bool fused0, bool pre_done,
+                           const double* dotv, double& acc) {
   using TM = Team<C>;
   const BatchLevel& Lv = d.lv[l];
   const Geo& g = Lv.g;
@@ -329,16 +491,20 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const TV* sK, TV w, const 
   };
   if (down) {
     if (fused0) {
-      b_fine2<C, TV, TV>(g, [&](long long ss, int c) { return wdb(c * n + ss); }, (const TV*)d.ET, d.mask, sK,
-                         [&](long long s, const TV* own, const TV* Au) {
+      b_fine2_op<C, TV, TV>(g, [&](int, int, long long ss, TV* v) {
+        v[0] = wdb(ss);
+        v[1] = wdb(n + ss);
+      }, (const TV*)d.ET, d.mask, sK, [&](long long s, const TV* own, const TV* Au) {
                            for (int c = 0; c < 2; ++c) r[c * n + s] = bv(c * n + s) - Au[c];
                          });
       TM::sync();
       return;
     }
     if (ns >= 1) {
-      for (long long q = TM::first(); q < nv; q += TM::stride()) x[q] = wdb(q);
-      TM::sync();
+      if (!pre_done) {
+        for (long long q = TM::first(); q < nv; q += TM::stride()) x[q] = wdb(q);
+        TM::sync();
+      }
       for (int s = 1; s < ns; ++s) {
         sweep_b(x, y);
         TV* t = x;
@@ -362,7 +528,7 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const TV* sK, TV w, const 
     }
     auto xbase = [&](long long q) { return fused0 ? wdb(q) : xb[q]; };
     if (ns >= 1) {
-      b_level_op<C, TV, TS>(d, l, e1, sK, [&](long long s, const TV* own, const TV* Au) {
+      auto last = [&](long long s, const TV* own, const TV* Au) {
         for (int c = 0; c < 2; ++c) {
           const long long q = c * n + s;
           const TV e = own[c] + w * Conv<TV>::from(__ldg(D + q)) * (r[q] - Au[c]);
@@ -370,7 +536,11 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const TV* sK, TV w, const 
           out[q] = v;
           if (dotv) acc += dotv[q] * (double)v;
         }
-      });
+      };
+      if (fused0)  // the correction is interpolated where it is read (b_vcycle skips the pass)
+        b_fine2_op<C, TV, TV>(g, ProlongIn<TV>{d.lv[1].g, (const TV*)d.lv[1].res}, (const TV*)d.ET, d.mask, sK, last);
+      else
+        b_level_op<C, TV, TS>(d, l, e1, sK, last);
     } else {
       for (long long q = TM::first(); q < nv; q += TM::stride()) {
         const TV v = Conv<TV>::from((double)xb[q] + (double)e1[q]);
@@ -382,16 +552,12 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const TV* sK, TV w, const 
   }
 }
 
-// z = V-cycle(r) into lv[0].res, r the FP64 PCG residual (read in the V-cycle's type); returns
-// this thread's part of r.z, which the caller sums over the team.
+// Levels [l0, l1) of a V-cycle downwards (smoothing, residual, restriction with the next level's first
+// sweep; pre_done: level l0's own first sweep was done that way) and upwards.  xcur: the levels' iterates.
 template <int C, typename TV, typename TD0, typename TS>
-EDGE_D double b_vcycle(const BatchDesc& d, const TV* sK, double omega, double* sb) {
-  using TM = Team<C>;
-  const int L = d.n_level;
-  TV* xcur[BATCH_MAXL];
-  const bool fused0 = d.sweeps[0] == 1;
+EDGE_D void b_down(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0, int l1, TV** xcur) {
   double acc = 0.0;
-  for (int l = 0; l < L; ++l) {
+  for (int l = l0; l < l1; ++l) {
     const BatchLevel& Lv = d.lv[l];
     TV* x = (TV*)Lv.xa;
     TV* y = (TV*)Lv.xb;
@@ -400,38 +566,73 @@ EDGE_D double b_vcycle(const BatchDesc& d, const TV* sK, double omega, double* s
     const TV w = Conv<TV>::from(omega * d.wscale[l]);
     if (l == 0)
       b_smooth_level<C, TV, TS, TD0, double>(d, l, sK, w, d.r64, nullptr, x, y, e1, e2, (TV*)Lv.r, nullptr, true,
-                                              fused0, nullptr, acc);
+                                              d.sweeps[0] == 1, false, nullptr, acc);
     else
       b_smooth_level<C, TV, TS, TV, TV>(d, l, sK, w, (const TV*)Lv.b, nullptr, x, y, e1, e2, (TV*)Lv.r, nullptr,
-                                        true, false, nullptr, acc);
+                                        true, false, d.sweeps[l] >= 1, nullptr, acc);
     xcur[l] = x;
-    b_restrict2<C, TV>(Lv.g, d.lv[l + 1].g, (const TV*)Lv.r, (TV*)d.lv[l + 1].b);
-    TM::sync();
+    const BatchLevel& Lc = d.lv[l + 1];
+    const bool j0 = l + 1 < d.n_level && d.sweeps[l + 1] >= 1;
+    b_restrict2<C, TV>(Lv.g, Lc.g, (const TV*)Lv.r, (TV*)Lc.b, (const TV*)Lc.dinv,
+                       Conv<TV>::from(omega * d.wscale[l + 1]), j0 ? (TV*)Lc.xa : nullptr);
+    Team<C>::sync();
   }
-  b_coarse2<C, TV>(d.lv[L].g, d.Ainv, d.nd, (const TV*)d.lv[L].b, (TV*)d.lv[L].res, sb);
-  TM::sync();
-  for (int l = L - 1; l >= 0; --l) {
+}
+template <int C, typename TV, typename TD0, typename TS>
+EDGE_D double b_up(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0, int l1, TV** xcur) {
+  double acc = 0.0;
+  for (int l = l1 - 1; l >= l0; --l) {
     const BatchLevel& Lv = d.lv[l];
+    const bool fused0 = l == 0 && d.sweeps[0] == 1;
     TV* e1 = (TV*)Lv.ea;
     TV* e2 = (TV*)Lv.eb;
     TV* x = nullptr;
     TV* y = nullptr;
-    b_prolong2<C, TV>(Lv.g, d.lv[l + 1].g, (const TV*)d.lv[l + 1].res, e1);
-    TM::sync();
+    if (!fused0) {
+      b_prolong2<C, TV>(Lv.g, d.lv[l + 1].g, (const TV*)d.lv[l + 1].res, e1);
+      Team<C>::sync();
+    }
     const TV w = Conv<TV>::from(omega * d.wscale[l]);
     if (l == 0)
       b_smooth_level<C, TV, TS, TD0, double>(d, l, sK, w, d.r64, xcur[l], x, y, e1, e2, (TV*)Lv.r, (TV*)Lv.res,
-                                              false, fused0, d.r64, acc);
+                                              false, fused0, false, d.r64, acc);
     else
       b_smooth_level<C, TV, TS, TV, TV>(d, l, sK, w, (const TV*)Lv.b, xcur[l], x, y, e1, e2, (TV*)Lv.r,
-                                        (TV*)Lv.res, false, false, nullptr, acc);
+                                        (TV*)Lv.res, false, false, false, nullptr, acc);
   }
   return acc;
 }
 
+// z = V-cycle(r) into lv[0].res, r the FP64 PCG residual (read in the V-cycle's type); returns
+// this thread's part of r.z, which the caller sums over the team.  Levels that one block covers with
+// a node per thread are smoothed by the team's first block alone: a step then ends in __syncthreads
+// (1.2 us a step) instead of a cluster barrier (2.7 to 4 us on 16 blocks).  The coarsest solve, a dense
+// product, is the whole team's.
 template <int C, typename TV, typename TD0, typename TS>
-EDGE_D void b_pcg_problem(const BatchDesc& d, const TV* sK, const double* sK64, double tol, int maxiter, double* sh,
-                          double* sb) {
+EDGE_D double b_vcycle(const BatchDesc& d, const FineK<TV>& sK, double omega, double* sb) {
+  using TM = Team<C>;
+  const int L = d.n_level;
+  TV* xcur[BATCH_MAXL];
+  int ls = L;  // levels [ls, L): the first block's
+  if constexpr (C > 1)
+    while (ls > 1 && d.lv[ls - 1].g.nx * d.lv[ls - 1].g.ny <= (int)blockDim.x) --ls;
+  b_down<C, TV, TD0, TS>(d, sK, omega, 0, ls, xcur);
+  if (ls < L) {
+    if (TM::rank() == 0) b_down<1, TV, TD0, TS>(d, sK, omega, ls, L, xcur);
+    TM::sync();
+  }
+  b_coarse2<C, TV>(d.lv[L].g, d.Ainv, d.nd, (const TV*)d.lv[L].b, (TV*)d.lv[L].res, sb);
+  TM::sync();
+  if (ls < L) {
+    if (TM::rank() == 0) b_up<1, TV, TD0, TS>(d, sK, omega, ls, L, xcur);
+    TM::sync();
+  }
+  return b_up<C, TV, TD0, TS>(d, sK, omega, 0, ls, xcur);
+}
+
+template <int C, typename TV, typename TD0, typename TS>
+EDGE_D void b_pcg_problem(const BatchDesc& d, const FineK<TV>& sK, const double* sK64, double tol, int maxiter,
+                          double* sh, double* sb) {
   using TM = Team<C>;
   const Geo& g = d.lv[0].g;
   const long long n = g.n, nv = 2 * n;
@@ -444,31 +645,32 @@ EDGE_D void b_pcg_problem(const BatchDesc& d, const TV* sK, const double* sK64, 
   double omega = d.keep_omega ? d.st->omega : d.omega0;
   const double min_omega = d.min_omega, d_omega = d.omega - d.min_omega;
   // r = b - A x (FP64)
-  b_fine2<C, double, double>(g, ArrIn<double>{x, n}, d.E64, d.mask, sK64,
+  b_fine2<C, double, double>(g, [&](long long s, int c) { return x[c * n + s]; }, d.E64, d.mask, sK64,
                              [&](long long s, const double* own, const double* Au) {
                                for (int c = 0; c < 2; ++c) r[c * n + s] = b[c * n + s] - Au[c];
                              });
   TM::sync();
-  const double bb = b_dot<C>(nv, b, b, sh);
+  int ph = 0;
+  const double bb = b_dot<C>(nv, b, b, sh, ph);
   int done = 0, iter = 0;
   double res = 0.0, rz = 0.0, rr = 0.0;
   if (bb == 0.0) done = 1;  // nothing to solve: residual 0, like a converged solve
   if (*d.chol_status) done = 3;
   while (!done) {
-    const double rz_new = TM::sum(b_vcycle<C, TV, TD0, TS>(d, sK, omega, sb), sh);
+    const double rz_new = TM::sum(b_vcycle<C, TV, TD0, TS>(d, sK, omega, sb), sh, ph);
     const double beta = iter == 0 ? 0.0 : rz_new / rz;
     for (long long k = TM::first(); k < nv; k += TM::stride())
       p[k] = iter == 0 ? (double)z[k] : (double)z[k] + beta * p[k];
     TM::sync();
     double acc = 0.0;
-    b_fine2<C, double, double>(g, ArrIn<double>{p, n}, d.E64, d.mask, sK64,
+    b_fine2<C, double, double>(g, [&](long long s, int c) { return p[c * n + s]; }, d.E64, d.mask, sK64,
                                [&](long long s, const double* own, const double* Au) {
                                  for (int c = 0; c < 2; ++c) {
                                    q[c * n + s] = Au[c];
                                    acc += own[c] * Au[c];
                                  }
                                });
-    const double pq = TM::sum(acc, sh);
+    const double pq = TM::sum(acc, sh, ph);
     const double alpha = rz_new / pq;
     double racc = 0.0;
     for (long long k = TM::first(); k < nv; k += TM::stride()) {
@@ -477,7 +679,7 @@ EDGE_D void b_pcg_problem(const BatchDesc& d, const TV* sK, const double* sK64, 
       r[k] = rv;
       racc += rv * rv;
     }
-    rr = TM::sum(racc, sh);
+    rr = TM::sum(racc, sh, ph);
     rz = rz_new;
     ++iter;
     const double R = sqrt(rr) / sqrt(bb);
@@ -516,10 +718,11 @@ template <typename TV, typename TD0, typename TS, int BT, int C>
 __global__ void __launch_bounds__(BT) k_batch_pcg(const BatchDesc* D, int nprob, unsigned* queue, double tol,
                                                   int maxiter, long long* tns) {
   using TM = Team<C>;
-  __shared__ double sh[33 + C];
+  __shared__ double sh[33 + 2 * C];
   __shared__ double sb[BATCH_COARSE_SMEM];
   __shared__ TV sK[64];
   __shared__ double sK64[64];
+  __shared__ KHat2<TV> sk2;
   __shared__ BatchDesc sd;
   __shared__ int s_idx;
   for (;;) {
@@ -540,9 +743,14 @@ __global__ void __launch_bounds__(BT) k_batch_pcg(const BatchDesc* D, int nprob,
       sK[k] = reinterpret_cast<const TV*>(sd.K0_T)[k];
       sK64[k] = sd.K0_64[k];
     }
+    if (threadIdx.x < 24) {
+      const double* src = &sd.k2.dg[0][0];
+      reinterpret_cast<TV*>(&sk2)[threadIdx.x] = (TV)src[threadIdx.x];
+    }
     __syncthreads();
+    const FineK<TV> fk{sK, sd.wht ? &sk2 : nullptr};
     const long long t0 = global_ns();
-    b_pcg_problem<C, TV, TD0, TS>(sd, sK, sK64, tol, maxiter, sh, sb);
+    b_pcg_problem<C, TV, TD0, TS>(sd, fk, sK64, tol, maxiter, sh, sb);
     TM::sync();
     if (tns && TM::first() == 0) {
       tns[2 * idx] = t0;

@@ -3790,8 +3790,8 @@ template <typename TV, typename TD0, typename TS, int BT> static int batch_clust
 // barrier and two trips to L2 whatever the size; a single block's barrier is nearly free), so the
 // smallest time T is sought for which the smallest sizes with time <= T fit.  Sizes are powers of two
 // up to 16 and their sum stays within the blocks that clusters of 16 could fill: powers of two then
-// pack into the GPCs.  24 problems: 285 -> 160 ms (every SM busy, problems end between 92 and 160 ms);
-// 8 and 17 problems: calls of 275 and 296 ms take 107 and 119.  Returns the sizes by queue position
+// pack into the GPCs.  24 problems: 285 -> 160 ms (every SM busy, problems end between 92 and 160 ms;
+// 137 with the marching fine operator).  Returns the sizes by queue position
 // and the predicted time of that choice.
 static double batch_sizes(const edge_batch& B, int budget, std::vector<int>& size) {
   static const int SZ[5] = {1, 2, 4, 8, 16};
@@ -4162,6 +4162,8 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
       d.ET = mixed ? (const void*)P.E32 : (const void*)P.E64;
       d.K0_64 = P.dK0b;
       d.K0_T = mixed ? (const void*)P.dK0bf : (const void*)P.dK0b;
+      d.wht = P.ei.wht ? 1 : 0;
+      d.k2 = P.ei.k2;
       d.b64 = P.b64;
       d.x64 = P.x64;
       d.r64 = P.r64;

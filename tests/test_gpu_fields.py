@@ -137,3 +137,31 @@ def test_coarsest_inverse_solves_a_two_level_system(nel):
     x, res = sv.solve(torch.as_tensor(p.f, device="cuda"), torch.as_tensor(E, device="cuda"), use_last=False)
     assert res < 1e-10 and sv.last_iters == p.solver.pcg_iters[-1]
     np.testing.assert_allclose(x.cpu().numpy(), ref, rtol=0, atol=1e-9 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("team", [1, 8])
+@pytest.mark.parametrize("box", [True, False])
+def test_batched_fine_operator_equals_the_per_problem_one(team, box, monkeypatch):
+    """Grids that end at, before and after the marching operator's 30-node columns, of few and many rows,
+    and an element matrix without the box structure (node-wise form): the batched FP64 solve takes the
+    per-problem solver's iterations and reaches its compliances.  Both stop at a relative residual of
+    1e-10, and a compliance's error is of the residual's second order: 1e-9 leaves the sums' roundings."""
+    import edge_to_b200 as eb
+    from edge_to_b200 import batch
+    if not box:
+        plain = eb.auto_stiffness
+
+        def anisotropic(x, E, nu):
+            K, D, B, A = plain(x, E, nu)
+            v = np.asarray(K) @ np.arange(1.0, 9.0) ** 2 / 40.0  # in K's range: rigid motions stay free
+            return K + 0.02 * np.outer(v, v), D, B, A
+        monkeypatch.setattr(eb, "auto_stiffness", anisotropic)
+    specs = [batch.random_spec(i, seed=9, nelx_range=(nx, nx), nely_range=(ny, ny))
+             for i, (nx, ny) in enumerate([(28, 4), (30, 16), (32, 40), (58, 6), (60, 62), (62, 9), (120, 90)])]
+    a = batch.BatchSIMP(specs, precision="fp64", tol=1e-10, maxiter=2000, n_threads=1)
+    c = batch.BatchSIMP(specs, precision="fp64", tol=1e-10, maxiter=2000, persistent=True, team=team)
+    a.step(2)
+    c.step(2)
+    for sp, ia, ic in zip(specs, a.items, c.items):
+        assert ia["pcg"] == ic["pcg"], sp["index"]
+        np.testing.assert_allclose(ic["comp"], ia["comp"], rtol=1e-9, atol=0)
