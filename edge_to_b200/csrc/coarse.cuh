@@ -32,18 +32,6 @@
 
 namespace edge {
 
-EDGE_HD double bnd_total3(int nb) { return nb == 3 ? 3.375 : nb == 2 ? 4.5 : nb == 1 ? 6.0 : 8.0; }
-EDGE_HD double bnd_total2(int nb) { return nb == 2 ? 2.25 : nb == 1 ? 3.0 : 4.0; }
-EDGE_HD double dist_w(int d) { return d == 0 ? 1.0 : d == 1 ? 0.5 : d == 2 ? 0.25 : 0.125; }
-EDGE_D int is_bnd(int i, int n) { return (i == 0 || i == n - 1) ? 1 : 0; }
-// 1 / bnd_total: the transfers multiply by these instead of dividing (a divide in FP64 is a
-// long instruction sequence; the results differ from the division by rounding only)
-template <typename T> EDGE_D T inv_bnd_total3(int nb) {
-  return nb == 3 ? T(1.0 / 3.375) : nb == 2 ? T(1.0 / 4.5) : nb == 1 ? T(1.0 / 6.0) : T(0.125);
-}
-template <typename T> EDGE_D T inv_bnd_total2(int nb) {
-  return nb == 2 ? T(1.0 / 2.25) : nb == 1 ? T(1.0 / 3.0) : T(0.25);
-}
 // arithmetic type of a transfer producing TO: FP64 for FP64 vectors, FP32 otherwise
 template <typename TO> struct TransferT {
   using type = float;

@@ -152,4 +152,39 @@ EDGE_D void grid_reduce_finish(double block_total, double* part, unsigned int* t
   }
 }
 
+// ------------------------------------------------------------------ transfer weights
+EDGE_HD double bnd_total3(int nb) { return nb == 3 ? 3.375 : nb == 2 ? 4.5 : nb == 1 ? 6.0 : 8.0; }
+EDGE_HD double bnd_total2(int nb) { return nb == 2 ? 2.25 : nb == 1 ? 3.0 : 4.0; }
+EDGE_HD double dist_w(int d) { return d == 0 ? 1.0 : d == 1 ? 0.5 : d == 2 ? 0.25 : 0.125; }
+EDGE_D int is_bnd(int i, int n) { return (i == 0 || i == n - 1) ? 1 : 0; }
+// 1 / bnd_total: the transfers multiply by these instead of dividing (a divide in FP64 is a
+// long instruction sequence; the results differ from the division by rounding only)
+template <typename T> EDGE_D T inv_bnd_total3(int nb) {
+  return nb == 3 ? T(1.0 / 3.375) : nb == 2 ? T(1.0 / 4.5) : nb == 1 ? T(1.0 / 6.0) : T(0.125);
+}
+template <typename T> EDGE_D T inv_bnd_total2(int nb) {
+  return nb == 2 ? T(1.0 / 2.25) : nb == 1 ? T(1.0 / 3.0) : T(0.25);
+}
+
+// ------------------------------------------------------------------ PCG device scalars
+struct PcgState {
+  double rz;      // r.z used by the current iteration's alpha / beta
+  double rz_new;  // r.z of the latest V-cycle
+  double pq;      // p.(A p)
+  double rr;      // r.r
+  double bb;      // f.f
+  double alpha, beta;
+  double res;     // ||r|| / ||f||
+  double omega;   // smoother weight for the next V-cycle
+  double tol, min_omega, d_omega;
+  double last_replace;      // ||r||/||f|| at the last true-residual replacement (mixed precision)
+  int iter, maxiter, done;  // done: 1 converged, 2 maxiter
+  int n_true;               // replacements made inside the iteration loop
+  // residual update folded into the next iteration's first fine launch (mixed path): pend =
+  // a search direction's product exists whose update is still to be applied; xa = the alpha
+  // of the solution update x32 += alpha p still to be applied (0: none)
+  int pend;
+  double xa;
+};
+
 }  // namespace edge

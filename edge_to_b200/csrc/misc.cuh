@@ -49,6 +49,27 @@ __global__ void k_slots_to_user(const Geo g, const TI* __restrict__ v, double* _
   for (int c = 0; c < g.dof; ++c) user[node * g.dof + c] = (double)Conv<double>::from(v[c * g.n + s]);
 }
 
+// User node order (reference numbering of the real nx_r x ny_r grid) <-> slots of a grid that
+// may be larger (padded): slots outside the real grid are zero.
+__global__ void k_user_to_slots_pad(const Geo g, int nxr, int nyr, const double* __restrict__ user,
+                                    double* __restrict__ v) {
+  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (s >= g.n) return;
+  const int i = (int)(s % g.pz), j = (int)(s / g.pz);
+  const bool ok = i < nxr && j < nyr;
+  const long long node = (long long)j * nxr + i;
+  for (int c = 0; c < 2; ++c) v[c * g.n + s] = ok ? user[node * 2 + c] : 0.0;
+}
+__global__ void k_slots_to_user_pad(const Geo g, int nxr, int nyr, const double* __restrict__ v,
+                                    double* __restrict__ user) {
+  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (s >= g.n) return;
+  const int i = (int)(s % g.pz), j = (int)(s / g.pz);
+  if (i >= nxr || j >= nyr) return;
+  const long long node = (long long)j * nxr + i;
+  for (int c = 0; c < 2; ++c) user[node * 2 + c] = v[c * g.n + s];
+}
+
 // Per-node constraint bits from the reference's per-DOF boolean array.
 __global__ void k_mask_from_user(const Geo g, const uint8_t* __restrict__ cons, uint8_t* __restrict__ mask) {
   EDGE_PDL_ENTRY();
@@ -248,27 +269,6 @@ __global__ void k_dot(long long n, const TA* __restrict__ a, const TB* __restric
   double bt = block_sum(acc, sh);
   grid_reduce_finish(bt, part, ticket, DotSink{dst});
 }
-
-// ------------------------------------------------------------------ PCG device scalars
-struct PcgState {
-  double rz;      // r.z used by the current iteration's alpha / beta
-  double rz_new;  // r.z of the latest V-cycle
-  double pq;      // p.(A p)
-  double rr;      // r.r
-  double bb;      // f.f
-  double alpha, beta;
-  double res;     // ||r|| / ||f||
-  double omega;   // smoother weight for the next V-cycle
-  double tol, min_omega, d_omega;
-  double last_replace;      // ||r||/||f|| at the last true-residual replacement (mixed precision)
-  int iter, maxiter, done;  // done: 1 converged, 2 maxiter
-  int n_true;               // replacements made inside the iteration loop
-  // residual update folded into the next iteration's first fine launch (mixed path): pend =
-  // a search direction's product exists whose update is still to be applied; xa = the alpha
-  // of the solution update x32 += alpha p still to be applied (0: none)
-  int pend;
-  double xa;
-};
 
 // x += alpha p ; r -= alpha q ; rr = r.r with alpha = rz_new / pq.  The finisher
 // updates res / omega / done as solvers/_multigrid_cuda.py:219-227 and moves rz_new to rz.

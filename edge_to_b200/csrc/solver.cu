@@ -1202,6 +1202,70 @@ static void launch_tail(Prob& P, int l0) {
   }
 }
 
+static SolveKind solve_kind(bool mixed, bool bf16) {
+  return !mixed ? SOLVE_FP64 : bf16 ? SOLVE_MIXED_BF16 : SOLVE_MIXED_FP32;
+}
+// The descriptor of a 2-D problem for the kernels of batch.cu.
+static void fill_desc(const Prob& P, bool mixed, bool bf16, BatchDesc& d) {
+  std::memset(&d, 0, sizeof(d));
+  d.n_level = P.n_level;
+  d.nd = P.nd;
+  d.keep_omega = (P.omega_carry && P.omega_started) ? 1 : 0;
+  for (int l = 0; l < BATCH_MAXL; ++l) {
+    d.sweeps[l] = l < P.n_level ? P.sweeps(l) : 0;
+    d.wscale[l] = std::pow(1.06, l);
+  }
+  d.omega = P.omega;
+  d.min_omega = P.min_omega;
+  d.omega0 = P.omega_carry ? P.omega : P.min_omega;
+  d.mask = P.mask;
+  d.E64 = P.E64;
+  d.ET = mixed ? (const void*)P.E32 : (const void*)P.E64;
+  d.K0_64 = P.dK0b;
+  d.K0_T = mixed ? (const void*)P.dK0bf : (const void*)P.dK0b;
+  d.wht = P.ei.wht ? 1 : 0;
+  d.k2 = P.ei.k2;
+  d.b64 = P.b64;
+  d.x64 = P.x64;
+  d.r64 = P.r64;
+  d.p64 = (double*)P.p;
+  d.q64 = (double*)P.q;
+  d.Ainv = P.Ainv;
+  d.st = P.st;
+  d.chol_status = P.chol_status;
+  for (int l = 0; l <= P.n_level; ++l) {
+    const Level& Lv = P.lv[l];
+    BatchLevel& bl = d.lv[l];
+    bl.g = Lv.g;
+    bl.b = Lv.b;
+    bl.xa = Lv.xa;
+    bl.xb = Lv.xb;
+    bl.r = Lv.r;
+    bl.ea = Lv.ea;
+    bl.eb = Lv.eb;
+    bl.res = Lv.res;
+    bl.S = (mixed && bf16 && Lv.S16) ? Lv.S16 : Lv.S;
+    bl.dinv = Lv.dinv;
+  }
+}
+
+// Whether the V-cycle below the fine level runs as one cluster launch (2-D, no second visits; while
+// launches are timed one by one they stay separate): as long as the cluster has a thread for every node
+// of level 1.  Time per PCG iteration, separate launches / one launch, FP64 (mixed): 64x32 elements 108
+// / 96 us (112 / 92), 120x40 107 / 100 (108 / 92), 160x96 139 / 128 (140 / 118); beyond, eight SMs are
+// too few: 240x120 129 / 270, and sixteen take 144.
+static bool vtail2_usable(const Prob& P) {
+  return P.dim == 2 && !P.bd && !P.prof && !(P.cycle_w && !P.w_levels.empty()) && P.n_level < BATCH_MAXL &&
+         (long long)P.lv[1].g.nx * P.lv[1].g.ny <= VTAIL_C * VTAIL_BT;
+}
+template <typename TV> static void vtail2(Prob& P) {
+  constexpr bool mixed = std::is_same<TV, float>::value;
+  BatchDesc d;
+  fill_desc(P, mixed, P.st_bf16, d);
+  P.nlaunch += vtail2_launch(solve_kind(mixed, P.st_bf16), d, &P.st->omega, P.stream);
+  KCHECK();
+}
+
 // Result in `out`; b and out have type T.  With dot_dst, the last fine sweep also
 // computes dotv . out (FP64 accumulation).
 // Whether the restriction from level l also runs level l+1's first sweep (mixed path, 3-D,
@@ -1329,18 +1393,22 @@ static void vcycle(Prob& P, int l, const T* b, T* out, const TV* dotv, double* d
     }
     const T* xcur = first ? x : out;
     Level& Lc = P.lv[l + 1];
-    restrict_to<T>(P, l, r);
-    vcycle<T, TD0, T>(P, l + 1, (const T*)Lc.b, (T*)Lc.res, (const T*)nullptr, nullptr, restrict_j0(P, l));
     T* e1 = (T*)Lv.ea;
     T* e2 = (T*)Lv.eb;
-    P.cur_cat = CAT_TRANSFER;
-    if (P.dim == 3)
-      launch(P, k_prolong3<T, T>, dim3(cdiv((long long)Lc.g.nz * Lc.g.nx, 256), Lc.g.ny), 256, 0, g, Lc.g,
-             (const T*)Lc.res, e1);
-    else
-      launch(P, k_prolong2<T, T>, dim3(cdiv(g.nx, 64), g.ny), 64, 0, g, Lc.g, (const T*)Lc.res, e1);
-    KCHECK();
-    P.cur_cat = CAT_VECTOR;
+    if (l == 0 && vtail2_usable(P)) {
+      vtail2<T>(P);
+    } else {
+      restrict_to<T>(P, l, r);
+      vcycle<T, TD0, T>(P, l + 1, (const T*)Lc.b, (T*)Lc.res, (const T*)nullptr, nullptr, restrict_j0(P, l));
+      P.cur_cat = CAT_TRANSFER;
+      if (P.dim == 3)
+        launch(P, k_prolong3<T, T>, dim3(cdiv((long long)Lc.g.nz * Lc.g.nx, 256), Lc.g.ny), 256, 0, g, Lc.g,
+               (const T*)Lc.res, e1);
+      else
+        launch(P, k_prolong2<T, T>, dim3(cdiv(g.nx, 64), g.ny), 64, 0, g, Lc.g, (const T*)Lc.res, e1);
+      KCHECK();
+      P.cur_cat = CAT_VECTOR;
+    }
     const bool last_visit = (vis == visits - 1);
     if (nsm >= 1) {
       for (int s = 0; s < nsm - 1; ++s) {
@@ -3700,87 +3768,17 @@ struct edge_batch {
 };
 
 namespace edge {
-// One persistent solve launch over the problems [off, off + cnt) of the queue order, on
-// `stream`, with at most `sm_budget` SMs' worth of blocks (0: as many as fit).
-template <typename TV, typename TD0, typename TS, int BT, int C>
-static void batch_go(Prob& P0, edge_batch& B, int off, int cnt, int qslot, int sm_budget, cudaStream_t stream,
-                     double tol, int maxiter) {
-  auto kern = k_batch_pcg<TV, TD0, TS, BT, C>;
-  if constexpr (C > 8) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  int dev = 0, sms = 0;
-  CK(cudaGetDevice(&dev));
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int budget = sm_budget > 0 ? std::min(sm_budget, sms) : sms;
-  const BatchDesc* D = B.d_desc + off;
-  long long* tns = B.d_tns + 2 * off;
-  if constexpr (C == 1) {
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT, 0));
-    const int grid = std::max(1, std::min(cnt, std::max(1, per_sm) * budget));
-    kern<<<grid, BT, 0, stream>>>(D, cnt, B.queue + qslot, tol, maxiter, tns);
-  } else {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C * sms);
-    cfg.blockDim = dim3(BT);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    CK(cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg));
-    const int fit = std::max(1, clusters * budget / sms);
-    const int teams = std::max(1, std::min(cnt, fit));
-    cfg.gridDim = dim3(C * teams);
-    CK(cudaLaunchKernelEx(&cfg, kern, D, cnt, B.queue + qslot, tol, maxiter, tns));
-  }
-  ++P0.nlaunch;
-  KCHECK();
-}
-template <typename TV, typename TD0, typename TS, int BT>
-static void batch_go_team(Prob& P0, edge_batch& B, int team, int off, int cnt, int qslot, int sm_budget,
-                          cudaStream_t stream, double tol, int maxiter) {
-  switch (team) {
-    case 2: batch_go<TV, TD0, TS, BT, 2>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
-    case 4: batch_go<TV, TD0, TS, BT, 4>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
-    case 8: batch_go<TV, TD0, TS, BT, 8>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
-    case 16: batch_go<TV, TD0, TS, BT, 16>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
-    default: batch_go<TV, TD0, TS, BT, 1>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter); break;
-  }
-}
-template <typename TV, typename TD0, typename TS>
-static void batch_group(Prob& P0, edge_batch& B, int threads, int team, int off, int cnt, int qslot, int sm_budget,
-                        cudaStream_t stream, double tol, int maxiter) {
-  if (threads == 1024)
-    batch_go_team<TV, TD0, TS, 1024>(P0, B, team, off, cnt, qslot, sm_budget, stream, tol, maxiter);
-  else if (threads == 256 && team == 1)
-    batch_go<TV, TD0, TS, 256, 1>(P0, B, off, cnt, qslot, sm_budget, stream, tol, maxiter);
-  else
-    batch_go_team<TV, TD0, TS, 512>(P0, B, team, off, cnt, qslot, sm_budget, stream, tol, maxiter);
-}
-// Clusters of 16 blocks of the solve kernel that the GPU holds at once (0: none).
-template <typename TV, typename TD0, typename TS, int BT> static int batch_clusters16() {
-  auto kern = k_batch_pcg<TV, TD0, TS, BT, 16>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 16;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(16);
-  cfg.blockDim = dim3(BT);
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return clusters;
+// Per-problem results of a batched call into contiguous arrays: residual, iterations, stop
+// reason, and the scalar the post-processing left in scal[2] (the compliance).
+__global__ void k_batch_gather(const BatchDesc* D, const double* const* scal, int nprob, double* res, double* comp,
+                               int* iters, int* done) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nprob) return;
+  const PcgState* st = D[i].st;
+  res[i] = st->res;
+  iters[i] = st->iter;
+  done[i] = st->done;
+  comp[i] = scal[i][2];
 }
 
 // Team sizes of a batch whose problems all fit on the GPU at once.  With teams of one size such a batch
@@ -3847,9 +3845,14 @@ static double batch_queue_time(const edge_batch& B, int sms) {
 // configured) are solved by single blocks in a second launch beside the teams' launch, on its
 // own share of the SMs (proportional to the groups' expected work), since a team's barriers
 // dominate a small problem's iteration.
-template <typename TV, typename TD0, typename TS>
-static void batch_launch(Prob& P0, edge_batch& B, int n, int n_large, double w_large, double w_small,
+static void batch_launch(SolveKind kind, Prob& P0, edge_batch& B, int n, int n_large, double w_large, double w_small,
                          cudaStream_t s, double tol, int maxiter) {
+  // the problems [off, off + cnt) of the queue order
+  auto go = [&](int threads, int team, int off, int cnt, int qslot, int sm_budget, cudaStream_t st) {
+    P0.nlaunch += batch_solve_launch(kind, threads, team, B.d_desc + off, cnt, B.queue + qslot, sm_budget, tol, maxiter,
+                                     B.d_tns + 2 * off, st);
+    KCHECK();
+  };
   if (!B.sized.empty()) {  // one launch per team size, side by side
     CK(cudaEventRecord(B.fork, s));
     int g = 0;
@@ -3858,7 +3861,7 @@ static void batch_launch(Prob& P0, edge_batch& B, int n, int n_large, double w_l
       while (e < n && B.sized[e] == B.sized[k]) ++e;
       cudaStream_t st = g == 0 ? s : B.side[g];
       if (g) CK(cudaStreamWaitEvent(st, B.fork, 0));
-      batch_group<TV, TD0, TS>(P0, B, B.threads, B.sized[k], k, e - k, g, 0, st, tol, maxiter);
+      go(B.threads, B.sized[k], k, e - k, g, 0, st);
       k = e;
     }
     for (int q = 1; q < g; ++q) {
@@ -3868,7 +3871,7 @@ static void batch_launch(Prob& P0, edge_batch& B, int n, int n_large, double w_l
     return;
   }
   if (B.team == 1 || n_large == n || n_large == 0) {
-    batch_group<TV, TD0, TS>(P0, B, B.threads, B.team, 0, n, 0, 0, s, tol, maxiter);
+    go(B.threads, B.team, 0, n, 0, 0, s);
     return;
   }
   int dev = 0, sms = 0;
@@ -3878,9 +3881,8 @@ static void batch_launch(Prob& P0, edge_batch& B, int n, int n_large, double w_l
   sm_large = std::max(B.team, std::min(sms - 1, sm_large)) / B.team * B.team;
   CK(cudaEventRecord(B.fork, s));
   CK(cudaStreamWaitEvent(B.side[0], B.fork, 0));
-  batch_group<TV, TD0, TS>(P0, B, B.threads, B.team, 0, n_large, 0, sm_large, s, tol, maxiter);
-  batch_group<TV, TD0, TS>(P0, B, B.small_threads, 1, n_large, n - n_large, 1, sms - sm_large, B.side[0], tol,
-                           maxiter);
+  go(B.threads, B.team, 0, n_large, 0, sm_large, s);
+  go(B.small_threads, 1, n_large, n - n_large, 1, sms - sm_large, B.side[0]);
   CK(cudaEventRecord(B.join[0], B.side[0]));
   CK(cudaStreamWaitEvent(s, B.join[0], 0));
 }
@@ -4075,15 +4077,7 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
     int clusters = 0, dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (!mixed)
-      clusters = B.threads == 1024 ? batch_clusters16<double, double, double, 1024>()
-                                   : batch_clusters16<double, double, double, 512>();
-    else if (bf16)
-      clusters = B.threads == 1024 ? batch_clusters16<float, __nv_bfloat16, __nv_bfloat16, 1024>()
-                                   : batch_clusters16<float, __nv_bfloat16, __nv_bfloat16, 512>();
-    else
-      clusters = B.threads == 1024 ? batch_clusters16<float, __nv_bfloat16, float, 1024>()
-                                   : batch_clusters16<float, __nv_bfloat16, float, 512>();
+    clusters = batch_clusters16(solve_kind(mixed, bf16), B.threads);
     std::vector<int> size;
     const double t = batch_sizes(B, std::min(16 * clusters, sms), size);
     if (t > 0.0 && t < batch_queue_time(B, sms)) {  // queue positions by size, then by cost
@@ -4145,47 +4139,7 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
       else
         CK(cudaMemsetAsync(P.x64, 0, (size_t)g.dof * g.n * sizeof(double), P.stream));
       mg_setup_prec(P);
-      BatchDesc& d = B.h_desc[k];
-      std::memset(&d, 0, sizeof(d));
-      d.n_level = P.n_level;
-      d.nd = P.nd;
-      d.keep_omega = (P.omega_carry && P.omega_started) ? 1 : 0;
-      for (int l = 0; l < BATCH_MAXL; ++l) {
-        d.sweeps[l] = l < P.n_level ? P.sweeps(l) : 0;
-        d.wscale[l] = std::pow(1.06, l);
-      }
-      d.omega = P.omega;
-      d.min_omega = P.min_omega;
-      d.omega0 = P.omega_carry ? P.omega : P.min_omega;
-      d.mask = P.mask;
-      d.E64 = P.E64;
-      d.ET = mixed ? (const void*)P.E32 : (const void*)P.E64;
-      d.K0_64 = P.dK0b;
-      d.K0_T = mixed ? (const void*)P.dK0bf : (const void*)P.dK0b;
-      d.wht = P.ei.wht ? 1 : 0;
-      d.k2 = P.ei.k2;
-      d.b64 = P.b64;
-      d.x64 = P.x64;
-      d.r64 = P.r64;
-      d.p64 = (double*)P.p;
-      d.q64 = (double*)P.q;
-      d.Ainv = P.Ainv;
-      d.st = P.st;
-      d.chol_status = P.chol_status;
-      for (int l = 0; l <= P.n_level; ++l) {
-        const Level& Lv = P.lv[l];
-        BatchLevel& bl = d.lv[l];
-        bl.g = Lv.g;
-        bl.b = Lv.b;
-        bl.xa = Lv.xa;
-        bl.xb = Lv.xb;
-        bl.r = Lv.r;
-        bl.ea = Lv.ea;
-        bl.eb = Lv.eb;
-        bl.res = Lv.res;
-        bl.S = (mixed && bf16 && Lv.S16) ? Lv.S16 : Lv.S;
-        bl.dinv = Lv.dinv;
-      }
+      fill_desc(P, mixed, bf16, B.h_desc[k]);
       B.h_scal[k] = P.scal;
     } catch (...) {
       P.stream = saved;
@@ -4203,12 +4157,7 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
     CK(cudaMemcpyAsync(B.d_scal, B.h_scal, n * sizeof(double*), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(B.queue, 0, edge_batch::NQ * sizeof(unsigned), s));
     CK(cudaEventRecord(B.ev[1], s));
-    if (!mixed)
-      batch_launch<double, double, double>(P0, B, n, n_large, w_large, w_small, s, tol, maxiter);
-    else if (bf16)
-      batch_launch<float, __nv_bfloat16, __nv_bfloat16>(P0, B, n, n_large, w_large, w_small, s, tol, maxiter);
-    else
-      batch_launch<float, __nv_bfloat16, float>(P0, B, n, n_large, w_large, w_small, s, tol, maxiter);
+    batch_launch(solve_kind(mixed, bf16), P0, B, n, n_large, w_large, w_small, s, tol, maxiter);
   } catch (...) {
     P0.stream = saved0;
     throw;

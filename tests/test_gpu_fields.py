@@ -165,3 +165,25 @@ def test_batched_fine_operator_equals_the_per_problem_one(team, box, monkeypatch
     for sp, ia, ic in zip(specs, a.items, c.items):
         assert ia["pcg"] == ic["pcg"], sp["index"]
         np.testing.assert_allclose(ic["comp"], ia["comp"], rtol=1e-9, atol=0)
+
+
+@pytest.mark.parametrize("nel,n_level", [((2, 2), 1), ((8, 4), 2), ((64, 30), 1), ((62, 64), 1), ((126, 126), 1),
+                                         ((128, 128), 2), ((48, 64), 4), ((128, 64), 6)])
+@pytest.mark.parametrize("n_smooth", [1, 3])
+def test_two_dimensional_cycle_below_the_fine_level(nel, n_level, n_smooth):
+    """Level 1 of four nodes up to the last size that runs as one launch (4,096 nodes) and the first that
+    does not, with levels of the whole cluster and of one block: the PCG takes the oracle's iterations
+    to rtol 1e-10 and reaches its solution, as it only does with the oracle's cycle."""
+    import torch
+    import edge_to_b200 as eb
+    p = topopt.mbb_problem(*nel, vf=0.4, mg_kwargs=dict(tol=1e-10, n_level=n_level, n_smooth=n_smooth, maxiter=600,
+                                                        variant="gpu"))
+    E = np.random.default_rng(4).uniform(0.3, 1.0, p.grid.n_el) ** 3
+    ref, _ = p.solver.solve(ops.assemble(p.grid, p.K0, E, p.cons), p.f, use_last=False)
+    mesh = eb.CuStructuredMesh2D(*nel, *map(float, nel), stiffness=lambda x: eb.auto_stiffness(x, 1.0, 0.3))
+    k = eb.CuStructuredStiffnessKernel(mesh)
+    k.add_constraints(p.cons)
+    sv = eb.CuMultiGrid(mesh, k, tol=1e-10, n_level=n_level, n_smooth=n_smooth, maxiter=600)
+    x, res = sv.solve(torch.as_tensor(p.f, device="cuda"), torch.as_tensor(E, device="cuda"), use_last=False)
+    assert res < 1e-10 and sv.last_iters == p.solver.pcg_iters[-1]
+    np.testing.assert_allclose(x.cpu().numpy(), ref, rtol=0, atol=1e-9 * np.abs(ref).max())
