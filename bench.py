@@ -3,7 +3,7 @@
 Workload (the reference's large 3-D demo size): hex8 cantilever 256x128x128
 (4,194,304 elements, 12,830,211 DOF), E0=1, Emin(void)=1e-9, nu=0.3, p=3, vf=0.1,
 r_min=2, x=0 face clamped, unit total downward load on the bottom edge at x=L,
-6-grid GMG (n_level=5, coarsest 675 DOF, FP64 Cholesky), PCG rtol 1e-6, move 0.2.
+6-grid GMG (n_level=5, coarsest 675 DOF, dense FP64 inverse), PCG rtol 1e-6, move 0.2.
 A step = one SIMP iteration (OC update + filter + SIMP law + GMG-PCG solve + compliance
 + sensitivity + filter transpose), warm-started like the reference.
 
