@@ -350,8 +350,32 @@ EDGE_D void oc_team(const BatchOcDesc& d, double move, double& last, int& steps,
   __shared__ OcBis sB;
   __shared__ int s_done, s_allz;
   unsigned rank = 0;
-  if constexpr (C > 1) rank = cg::this_cluster().block_rank();
+  if constexpr (C > 1) {
+    rank = cg::this_cluster().block_rank();
+    // a peer's shared memory may be written once that block has started: arrive here, wait below, so
+    // that the elements' loads hide the barrier
+    cg::this_cluster().barrier_arrive();
+  }
   const long long i0 = rank * (long long)BT + threadIdx.x, T = (long long)C * BT;
+  double rr[REG], oo[REG];
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < REG; ++q) {
+    const long long i = i0 + q * T;
+    rr[q] = oo[q] = 0.0;
+    if (i < d.n) {
+      rr[q] = d.rho[i];
+      const double o = oc_raw(rr[q], d.dr[i], d.A);
+      any = any || o != 0.0;
+      oo[q] = fmax(1e-12, o);
+    }
+  }
+  for (long long i = i0 + REG * T; i < d.n; i += T) {
+    const double o = oc_raw(d.rho[i], d.dr[i], d.A);
+    any = any || o != 0.0;
+    d.ocp[i] = fmax(1e-12, o);
+  }
+  if constexpr (C > 1) cg::this_cluster().barrier_wait();
   int buf = 0;
   // team sums of v[0..15] -> ssum (the same in every block)
   auto team_sum = [&](double v[16]) {
@@ -371,24 +395,6 @@ EDGE_D void oc_team(const BatchOcDesc& d, double move, double& last, int& steps,
       __syncthreads();
     }
   };
-  double rr[REG], oo[REG];
-  bool any = false;
-#pragma unroll
-  for (int q = 0; q < REG; ++q) {
-    const long long i = i0 + q * T;
-    rr[q] = oo[q] = 0.0;
-    if (i < d.n) {
-      rr[q] = d.rho[i];
-      const double o = oc_raw(rr[q], d.dr[i], d.A);
-      any = any || o != 0.0;
-      oo[q] = fmax(1e-12, o);
-    }
-  }
-  for (long long i = i0 + REG * T; i < d.n; i += T) {
-    const double o = oc_raw(d.rho[i], d.dr[i], d.A);
-    any = any || o != 0.0;
-    d.ocp[i] = fmax(1e-12, o);
-  }
   if (threadIdx.x == 0) {
     sB = oc_start();
     s_done = 0;
