@@ -450,6 +450,8 @@ k_st3_apply_d(const Geo g, const T* __restrict__ u, const TS* __restrict__ S, Ep
   double dacc = 0.0;
   const int k = (int)(s % g.pz), i = (int)((s / g.pz) % g.nx), j = (int)(s / g.plane);
   const bool valid = s0 < n && k < g.nz;
+  T own[3], Au[3];
+  typename Epi::Pre pe{};
   if (w < ST3D_WARPS - 1) {
     const int nb = 14 + w, dz = nb % 3 - 1, dx = (nb / 3) % 3 - 1, dy = nb / 9 - 1;
     const long long off = (long long)dy * g.plane + (long long)dx * g.pz + dz;
@@ -477,11 +479,10 @@ k_st3_apply_d(const Geo g, const T* __restrict__ u, const TS* __restrict__ S, Ep
     for (int c = 0; c < 3; ++c)
       sA[w][c][lane] = (cu[c * 3] * vu[0] + cu[c * 3 + 1] * vu[1] + cu[c * 3 + 2] * vu[2]) +
                        (cl[c] * vl[0] + cl[3 + c] * vl[1] + cl[6 + c] * vl[2]);
-    __syncthreads();
   } else {
     epi.init();
-    const typename Epi::Pre pe = epi.pre(s);  // s is clamped into the array
-    T own[3], cc[6], Au[3];
+    pe = epi.pre(s);  // s is clamped into the array
+    T cc[6];
 #pragma unroll
     for (int c = 0; c < 3; ++c) own[c] = __ldg(u + c * n + s);
 #pragma unroll
@@ -489,7 +490,9 @@ k_st3_apply_d(const Geo g, const T* __restrict__ u, const TS* __restrict__ S, Ep
     Au[0] = cc[0] * own[0] + cc[1] * own[1] + cc[2] * own[2];
     Au[1] = cc[1] * own[0] + cc[3] * own[1] + cc[4] * own[2];
     Au[2] = cc[2] * own[0] + cc[4] * own[1] + cc[5] * own[2];
-    __syncthreads();
+  }
+  __syncthreads();  // one barrier that every warp reaches
+  if (w == ST3D_WARPS - 1) {
 #pragma unroll
     for (int d = 0; d < ST3D_WARPS - 1; ++d)
 #pragma unroll

@@ -1,5 +1,5 @@
-"""Barriers of the cluster kernels, checked on their source: a fault here would be undefined behaviour
-on the device, not a wrong value."""
+"""Barriers of the cluster kernels and of the block kernels with a role per warp, checked on their
+source: a fault here would be undefined behaviour on the device, not a wrong value."""
 import os
 import re
 
@@ -38,3 +38,12 @@ def test_peer_shared_memory_is_addressed_behind_a_cluster_barrier():
     assert src.count("map_shared_rank") == 2 and kern.count("map_shared_rank") == 1
     assert kern.index("TM::sync()") < kern.index("map_shared_rank") < kern.index("b_pcg_problem")
     assert "::sum(" not in body(src, "k_vtail2")
+
+
+def test_stencil_warps_meet_at_one_barrier():
+    """k_st3_apply_d gives its warps different work; __syncthreads() is defined only where every thread of
+    the block reaches the same one, so none may stand inside a branch."""
+    b = body(source("coarse.cuh"), "k_st3_apply_d")
+    assert b.count("__syncthreads()") == 1
+    before = b[:b.index("__syncthreads()")]
+    assert before.count("{") == before.count("}")
