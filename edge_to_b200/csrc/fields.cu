@@ -4,7 +4,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 #include <type_traits>
 
@@ -513,11 +512,8 @@ int oc_launch(long long n, const double* rho, const double* dr, double A, double
   cfg.stream = stream;
   cfg.attrs = at;
   if (n <= OC_CLUSTER_MAX) {
-    static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
-    if (!attr.load()) {
-      if (cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
-      attr = true;
-    }
+    // on every call: the attribute belongs to the current device's context, not to the process
+    if (cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = OC_TEAM;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -1542,13 +1538,10 @@ int spd_inverse(double* A, int nd, double* Ainv, double* work, int* status, cuda
   const int np = inv_padded(nd), nt = np / INV_B;
   double *Rt = work, *Wt = Rt + (long long)INV_B * np, *P0 = Wt + (long long)INV_B * np, *P1 = P0 + INV_B * INV_B;
   constexpr int psmem = 2 * INV_B * INV_LD * 8, usmem = 2 * INV_B * INV_B * 8;
-  static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
-  if (!attr.load()) {
-    if (cudaFuncSetAttribute(k_inv_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_inv_update, cudaFuncAttributeMaxDynamicSharedMemorySize, usmem) != cudaSuccess)
-      return 0;
-    attr = true;
-  }
+  // on every call: the attributes belong to the current device's context, not to the process
+  if (cudaFuncSetAttribute(k_inv_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_inv_update, cudaFuncAttributeMaxDynamicSharedMemorySize, usmem) != cudaSuccess)
+    return 0;
   k_inv_start<<<1, INV_T, 0, stream>>>(A, nd, np, P0, status);
   int n = 1;
   for (int K = 0; K < nt; ++K) {

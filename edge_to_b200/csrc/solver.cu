@@ -10,7 +10,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -647,11 +646,8 @@ template <typename T, class Epi, int BX, int NS>
 static void fine3_tma_launch(Prob& P, const T* u, const T* E, Epi epi, double* dot_dst) {
   const Geo& g = P.g0;
   constexpr int smem = tma_smem_bytes<T, BX, NS>();
-  static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
-  if (!attr.load()) {
-    CK(cudaFuncSetAttribute(k_fine3_tma<T, Epi, BX, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  // on every launch: the attribute belongs to the current device's context, not to the process
+  CK(cudaFuncSetAttribute(k_fine3_tma<T, Epi, BX, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const unsigned tz = cdiv(g.nz, 15), tx = cdiv(g.nx, 2 * BX - 1);
   const long long want = 148LL * P.blocks_per_sm;
   long long chunks = std::max<long long>(1, (want + (long long)tz * tx - 1) / ((long long)tz * tx));
@@ -667,11 +663,7 @@ template <class Epi, int BX, int NS, int MINB>
 static void fine3_pk_launch(Prob& P, const float* u, const float* E, Epi epi, double* dot_dst) {
   const Geo& g = P.g0;
   constexpr int smem = pk_smem_bytes<BX, NS>();
-  static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
-  if (!attr.load()) {
-    CK(cudaFuncSetAttribute(k_fine3_pk<Epi, BX, NS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  CK(cudaFuncSetAttribute(k_fine3_pk<Epi, BX, NS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const unsigned tz = cdiv(g.nz, 15), tx = cdiv(g.nx, 4 * BX - 1);
   const long long want = 148LL * P.blocks_per_sm;
   long long chunks = std::max<long long>(1, (want + (long long)tz * tx - 1) / ((long long)tz * tx));
@@ -788,11 +780,7 @@ static void fine3_cube_go(Prob& P, const float* in0, const void* in1, const void
   const Geo& g = P.g0;
   constexpr int smem = cube_smem_bytes<BX, NS, SE, IN>();
   static_assert(smem <= 227 * 1024, "cube kernel stage ring exceeds shared memory");
-  static std::atomic<bool> attr{false};  // setting the attribute twice is harmless
-  if (!attr.load()) {
-    CK(cudaFuncSetAttribute(k_fine3_cube<SE, BX, NS, MINB, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  CK(cudaFuncSetAttribute(k_fine3_cube<SE, BX, NS, MINB, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const CUtensorMap& m0 = pk_map<BX>(P, in0, 0);
   const CUtensorMap& m0b = xa.in0b ? pk_map<BX>(P, xa.in0b, 0) : m0;
   const CUtensorMap& m1 = IN::kN >= 2 ? in_map<BX>(P, in1, IN::kT1) : m0;
