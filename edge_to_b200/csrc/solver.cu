@@ -1238,13 +1238,20 @@ static void fill_desc(const Prob& P, bool mixed, bool bf16, BatchDesc& d) {
 }
 
 // Whether the V-cycle below the fine level runs as one cluster launch (2-D, no second visits; while
-// launches are timed one by one they stay separate): as long as the cluster has a thread for every node
-// of level 1.  Time per PCG iteration, separate launches / one launch, FP64 (mixed): 64x32 elements 108
-// / 96 us (112 / 92), 120x40 107 / 100 (108 / 92), 160x96 139 / 128 (140 / 118); beyond, eight SMs are
-// too few: 240x120 129 / 270, and sixteen take 144.
+// launches are timed one by one they stay separate).  The launch runs on eight SMs, so it has to be
+// small in two respects.  Level 1: a thread of the cluster for every node (64x32 elements, FP64: 96 us
+// per PCG iteration against 108 with separate launches, 160x96 128 / 139; 240x120 270 / 129).  The
+// coarsest DOFs, whose dense product grows with their square (FP64, three sweeps, us per iteration in
+// one launch / separate: 162 DOFs 93 / 105, 242 97 / 104, 306 80 / 79, 578 93 / 81, 1,250 195 / 84, 2,048
+// 334 / 82; 8,192 7,231 / 188).  The lines lie where both take the same time: 240 in FP64, 320 in mixed
+// precision (338 DOFs 65.5 / 67.6 with one sweep, 100 / 112 with three; 546 75 / 68, 112 / 113); with one
+// sweep in FP64 a level saves too few launches beyond 128 (128 DOFs 70.9 / 70.9, 200 59.4 / 57.5).  With one
+// coarse level there is nothing between the transfers to save (306 DOFs 40 / 36).
 static bool vtail2_usable(const Prob& P) {
-  return P.dim == 2 && !P.bd && !P.prof && !(P.cycle_w && !P.w_levels.empty()) && P.n_level < BATCH_MAXL &&
-         (long long)P.lv[1].g.nx * P.lv[1].g.ny <= VTAIL_C * VTAIL_BT;
+  if (P.dim != 2 || P.bd || P.prof || (P.cycle_w && !P.w_levels.empty()) || P.n_level < 2 || P.n_level >= BATCH_MAXL)
+    return false;
+  const int nd_max = P.prec != EDGE_FP64 ? 320 : P.sweeps(1) >= 2 ? 240 : 128;
+  return (long long)P.lv[1].g.nx * P.lv[1].g.ny <= VTAIL_C * VTAIL_BT && P.nd <= nd_max;
 }
 template <typename TV> static void vtail2(Prob& P) {
   constexpr bool mixed = std::is_same<TV, float>::value;

@@ -187,3 +187,46 @@ def test_two_dimensional_cycle_below_the_fine_level(nel, n_level, n_smooth):
     x, res = sv.solve(torch.as_tensor(p.f, device="cuda"), torch.as_tensor(E, device="cuda"), use_last=False)
     assert res < 1e-10 and sv.last_iters == p.solver.pcg_iters[-1]
     np.testing.assert_allclose(x.cpu().numpy(), ref, rtol=0, atol=1e-9 * np.abs(ref).max())
+
+
+def _launches_per_iteration(nel, n_level, n_smooth, precision):
+    import torch
+    import edge_to_b200 as eb
+    from edge_to_b200 import _lib
+    mesh = eb.CuStructuredMesh2D(*nel, *map(float, nel), stiffness=lambda x: eb.auto_stiffness(x, 1.0, 0.3))
+    k = eb.CuStructuredStiffnessKernel(mesh)
+    left = np.arange(nel[1] + 1) * (nel[0] + 1)
+    k.add_constraints(np.concatenate([2 * left, 2 * left + 1]))
+    f = np.zeros(k.shape[0])
+    f[-1] = -1.0
+    f, E = torch.as_tensor(f, device="cuda"), torch.full((int(np.prod(nel)),), 0.5, dtype=torch.float64, device="cuda")
+    last = None
+    for its in range(2, 12):
+        sv = eb.CuMultiGrid(mesh, k, tol=1e-300, n_level=n_level, n_smooth=n_smooth, maxiter=its, precision=precision,
+                            tune_sweeps=False)
+        counts = []
+        for _ in range(3):  # the first solve may tune
+            n = ctypes.c_longlong()
+            sv.solve(f, E, use_last=False)
+            _lib.call("edge_launch_count", k.handle, ctypes.byref(n))
+            counts.append(n.value)
+        assert sv.last_iters == its
+        now = counts[2] - counts[1], sv.stats()["true_residuals"]
+        if last and last[1] == now[1]:  # no residual replacement (mixed precision) in the added iteration
+            return now[0] - last[0]
+        last = now
+    raise AssertionError("every iteration replaced the residual")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_large_coarsest_levels_stay_out_of_the_one_launch_cycle(precision):
+    """The one-launch cycle runs on eight SMs, the dense product of a large coarsest level needs all of
+    them (8,192 coarsest DOFs took 7.2 ms per iteration in one launch, 0.19 with separate ones).  A level
+    between the transfers costs 2 n_smooth + 3 launches of its own where the cycle is separate, none where
+    it is one launch."""
+    for ns in (1, 3):
+        one = _launches_per_iteration((96, 96), 1, ns, precision)    # 4,802 coarsest DOFs
+        two = _launches_per_iteration((96, 96), 2, ns, precision)    # 1,250
+        assert two - one == 2 * ns + 3
+    three = _launches_per_iteration((64, 64), 3, 3, precision)       # 162 coarsest DOFs: one launch
+    assert three < two
