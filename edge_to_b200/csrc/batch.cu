@@ -16,9 +16,9 @@
 // nodes (the team's threads striding over them) followed by a team barrier (__syncthreads, or
 // the cluster barrier with its release/acquire ordering), which makes the team's global writes
 // visible to its next step (data written inside the launch is read with plain loads, never
-// through the read-only path); inner products are sums in a fixed order (per block, then over
-// the cluster's blocks through distributed shared memory), so a problem's result does not
-// depend on the team that solved it or on the other problems.  The PCG loop is bounded by
+// through the read-only path); inner products are sums in an order that does not depend on the
+// team's size (TeamSum), and every other step is node by node, so a problem's result, bit for bit,
+// depends neither on the team that solved it nor on the other problems (for a given block size).  The PCG loop is bounded by
 // maxiter; the queue counter is the only state shared between teams and nothing waits on it
 // (the cluster barrier only joins the blocks of one team, which run together).
 #include "batch.cuh"
@@ -32,12 +32,7 @@ namespace edge {
 
 constexpr int BATCH_COARSE_SMEM = 1024;  // coarsest right-hand sides up to this size are staged in shared memory
 
-// The blocks that solve one problem together.  sum(): the team-wide FP64 sum of a per-thread
-// value in a fixed order, returned to every thread, and a team barrier; `sh` holds 33 + 2 C doubles of
-// shared memory, `ph` alternates between its two halves from sum to sum (alike in every thread).
-// Each block writes its sum into every block's shared memory, so that after one cluster barrier all
-// threads read locally; all threads reading rank 0's C values through distributed shared memory
-// queued up there, and took a second barrier.
+// The blocks that solve one problem together.
 template <int C> struct Team {
   static EDGE_D unsigned rank() {
     if constexpr (C == 1) return 0;
@@ -49,24 +44,48 @@ template <int C> struct Team {
     if constexpr (C == 1) __syncthreads();
     else cooperative_groups::this_cluster().sync();
   }
-  static EDGE_D double sum(double v, double* sh, int& ph) {
-    double r = block_sum(v, sh);  // valid in every lane of warp 0 of each block
-    if constexpr (C == 1) {
-      if (threadIdx.x == 0) sh[32] = r;
-      __syncthreads();
-      r = sh[32];
-      return r;  // sh is written again only behind block_sum's barrier
-    } else {
-      auto cl = cooperative_groups::this_cluster();
-      double* half = sh + 33 + ph * C;
-      if (threadIdx.x < C) *cl.map_shared_rank(half + rank(), threadIdx.x) = r;
-      cl.sync();
-      double t = 0.0;
-#pragma unroll
-      for (int k = 0; k < C; ++k) t += half[k];
-      ph ^= 1;  // this half is written again two sums from now, behind the next sum's barrier
-      return t;
+};
+
+// Team-wide FP64 sums, returned to every thread; the sum is also a team barrier.  Team sizes are chosen
+// by what else is solved beside a problem, so the order of a sum must not follow them: the terms are
+// those of TEAM_MAX virtual blocks whatever the team's size C (term k belongs to thread k mod BT of
+// virtual block (k / BT) mod TEAM_MAX), a block of the team adds up its TEAM_MAX / C virtual blocks one
+// after the other, and the TEAM_MAX block sums are added in their order.  A thread handles the terms that
+// a plain stride over the team would give it.
+//
+// pass(first, step, acc) adds the terms first, first + step, ... to acc.  sh: TeamSum<C>::SH doubles of
+// shared memory; ph alternates between the two halves of the block sums from sum to sum (alike in every
+// thread).  Each block writes its block sums into every block's shared memory, so that after one
+// cluster barrier all threads read locally.
+constexpr int TEAM_MAX = 16;
+template <int C> struct TeamSum {
+  static constexpr int PER = TEAM_MAX / C;      // virtual blocks of a block
+  static constexpr int SH = PER * 32 + 2 * TEAM_MAX;  // their warps' sums, the block sums
+  template <class Pass> static EDGE_D double run(Pass&& pass, double* sh, int& ph) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, BT = blockDim.x;
+    const int rank = (int)Team<C>::rank();
+    double* half = sh + PER * 32 + ph * TEAM_MAX;
+    for (int q = 0; q < PER; ++q) {
+      double acc = 0.0;
+      pass((rank + q * C) * BT + (int)threadIdx.x, TEAM_MAX * BT, acc);
+      acc = warp_sum(acc);
+      if (lane == 0) sh[q * 32 + wid] = acc;  // read last before the previous sum's team barrier
     }
+    __syncthreads();
+    for (int q = wid; q < PER; q += nw) {
+      const double r = warp_sum(lane < nw ? sh[q * 32 + lane] : 0.0);
+      if constexpr (C == 1) {
+        if (lane == 0) half[q] = r;
+      } else {
+        if (lane < C) *cooperative_groups::this_cluster().map_shared_rank(half + rank + q * C, lane) = r;
+      }
+    }
+    Team<C>::sync();
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < TEAM_MAX; ++k) t += half[k];
+    ph ^= 1;  // this half is written again two sums from now, behind the next sum's barrier
+    return t;
   }
 };
 
@@ -85,9 +104,10 @@ template <int C> struct Team {
 // form), and marching with the full matrix in this order of sums spills at 1024 threads (354 ms a solve of
 // those 8 problems, 171 with this form).
 template <int C, typename T, typename TE, class UIn, class F>
-EDGE_D void b_fine2(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, const T* sK, F&& epi) {
+EDGE_D void b_fine2(const Geo& g, UIn uin, const TE* E, const uint8_t* mask, const T* sK, F&& epi,
+                    int first = Team<C>::first(), int step = Team<C>::stride()) {
   const int nn = g.nx * g.ny;
-  for (int t = Team<C>::first(); t < nn; t += Team<C>::stride()) {
+  for (int t = first; t < nn; t += step) {
     const int i = t % g.nx, j = t / g.nx;
     const long long s = g.slot2(i, j);
     T U[3][3][2];
@@ -408,9 +428,9 @@ EDGE_D void b_coarse2(const Geo& g, const double* Ainv, int nd, const T* b, T* x
 
 template <int C, typename TA, typename TB>
 EDGE_D double b_dot(long long nv, const TA* a, const TB* b, double* sh, int& ph) {
-  double acc = 0.0;
-  for (long long q = Team<C>::first(); q < nv; q += Team<C>::stride()) acc += (double)a[q] * (double)b[q];
-  return Team<C>::sum(acc, sh, ph);
+  return TeamSum<C>::run([&](int first, int step, double& acc) {
+    for (long long q = first; q < nv; q += step) acc += (double)a[q] * (double)b[q];
+  }, sh, ph);
 }
 
 // One application of level l's operator (fine: the element operator in TV; coarser: the
@@ -429,11 +449,10 @@ EDGE_D void b_level_op(const BatchDesc& d, int l, const TV* u, const FineK<TV>& 
 // one pass (the operator's input w Dinv b computed where it is read, x never stored: fused0).
 // up (after the interpolation into e1): ns - 1 sweeps on the correction, then
 // out = xb + (e + w Dinv (r - A e)) with xb the down pass's x (recomputed as w Dinv b when
-// fused0); with dot, acc += dotv . out (the PCG's r.z) per thread.
+// fused0).
 template <int C, typename TV, typename TS, typename TD, typename TB>
 EDGE_D void b_smooth_level(const BatchDesc& d, int l, const FineK<TV>& sK, TV w, const TB* b, const TV* xb, TV*& x, TV*& y,
-                           TV*& e1, TV*& e2, TV* r, TV* out, bool down, bool fused0, bool pre_done,
-                           const double* dotv, double& acc) {
+                           TV*& e1, TV*& e2, TV* r, TV* out, bool down, bool fused0, bool pre_done) {
   using TM = Team<C>;
   const BatchLevel& Lv = d.lv[l];
   const Geo& g = Lv.g;
@@ -503,9 +522,7 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const FineK<TV>& sK, TV w,
         for (int c = 0; c < 2; ++c) {
           const long long q = c * n + s;
           const TV e = own[c] + w * Conv<TV>::from(__ldg(D + q)) * (r[q] - Au[c]);
-          const TV v = xbase(q) + e;
-          out[q] = v;
-          if (dotv) acc += dotv[q] * (double)v;
+          out[q] = xbase(q) + e;
         }
       };
       if (fused0)  // the correction is interpolated where it is read (b_vcycle skips the pass)
@@ -513,13 +530,9 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const FineK<TV>& sK, TV w,
       else
         b_level_op<C, TV, TS>(d, l, e1, sK, last);
     } else {
-      for (long long q = TM::first(); q < nv; q += TM::stride()) {
-        const TV v = Conv<TV>::from((double)xb[q] + (double)e1[q]);
-        out[q] = v;
-        if (dotv) acc += dotv[q] * (double)v;
-      }
+      for (long long q = TM::first(); q < nv; q += TM::stride()) out[q] = Conv<TV>::from((double)xb[q] + (double)e1[q]);
     }
-    if (!dotv) TM::sync();  // with dot, the team sum that follows is the barrier
+    TM::sync();
   }
 }
 
@@ -527,7 +540,6 @@ EDGE_D void b_smooth_level(const BatchDesc& d, int l, const FineK<TV>& sK, TV w,
 // sweep; pre_done: level l0's own first sweep was done that way) and upwards.  xcur: the levels' iterates.
 template <int C, typename TV, typename TD0, typename TS>
 EDGE_D void b_down(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0, int l1, TV** xcur) {
-  double acc = 0.0;
   for (int l = l0; l < l1; ++l) {
     const BatchLevel& Lv = d.lv[l];
     TV* x = (TV*)Lv.xa;
@@ -537,10 +549,10 @@ EDGE_D void b_down(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0
     const TV w = Conv<TV>::from(omega * d.wscale[l]);
     if (l == 0)
       b_smooth_level<C, TV, TS, TD0, double>(d, l, sK, w, d.r64, nullptr, x, y, e1, e2, (TV*)Lv.r, nullptr, true,
-                                              d.sweeps[0] == 1, false, nullptr, acc);
+                                              d.sweeps[0] == 1, false);
     else
       b_smooth_level<C, TV, TS, TV, TV>(d, l, sK, w, (const TV*)Lv.b, nullptr, x, y, e1, e2, (TV*)Lv.r, nullptr,
-                                        true, false, d.sweeps[l] >= 1, nullptr, acc);
+                                        true, false, d.sweeps[l] >= 1);
     xcur[l] = x;
     const BatchLevel& Lc = d.lv[l + 1];
     const bool j0 = l + 1 < d.n_level && d.sweeps[l + 1] >= 1;
@@ -550,8 +562,7 @@ EDGE_D void b_down(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0
   }
 }
 template <int C, typename TV, typename TD0, typename TS>
-EDGE_D double b_up(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0, int l1, TV** xcur) {
-  double acc = 0.0;
+EDGE_D void b_up(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0, int l1, TV** xcur) {
   for (int l = l1 - 1; l >= l0; --l) {
     const BatchLevel& Lv = d.lv[l];
     const bool fused0 = l == 0 && d.sweeps[0] == 1;
@@ -566,21 +577,19 @@ EDGE_D double b_up(const BatchDesc& d, const FineK<TV>& sK, double omega, int l0
     const TV w = Conv<TV>::from(omega * d.wscale[l]);
     if (l == 0)
       b_smooth_level<C, TV, TS, TD0, double>(d, l, sK, w, d.r64, xcur[l], x, y, e1, e2, (TV*)Lv.r, (TV*)Lv.res,
-                                              false, fused0, false, d.r64, acc);
+                                              false, fused0, false);
     else
       b_smooth_level<C, TV, TS, TV, TV>(d, l, sK, w, (const TV*)Lv.b, xcur[l], x, y, e1, e2, (TV*)Lv.r,
-                                        (TV*)Lv.res, false, false, false, nullptr, acc);
+                                        (TV*)Lv.res, false, false, false);
   }
-  return acc;
 }
 
-// z = V-cycle(r) into lv[0].res, r the FP64 PCG residual (read in the V-cycle's type); returns
-// this thread's part of r.z, which the caller sums over the team.  Levels that one block covers with
+// z = V-cycle(r) into lv[0].res, r the FP64 PCG residual (read in the V-cycle's type).  Levels that one block covers with
 // a node per thread are smoothed by the team's first block alone: a step then ends in __syncthreads
 // (1.2 us a step) instead of a cluster barrier (2.7 to 4 us on 16 blocks).  The coarsest solve, a dense
 // product, is the whole team's.
 template <int C, typename TV, typename TD0, typename TS>
-EDGE_D double b_vcycle(const BatchDesc& d, const FineK<TV>& sK, double omega, double* sb) {
+EDGE_D void b_vcycle(const BatchDesc& d, const FineK<TV>& sK, double omega, double* sb) {
   using TM = Team<C>;
   const int L = d.n_level;
   TV* xcur[BATCH_MAXL];
@@ -598,7 +607,7 @@ EDGE_D double b_vcycle(const BatchDesc& d, const FineK<TV>& sK, double omega, do
     if (TM::rank() == 0) b_up<1, TV, TD0, TS>(d, sK, omega, ls, L, xcur);
     TM::sync();
   }
-  return b_up<C, TV, TD0, TS>(d, sK, omega, 0, ls, xcur);
+  b_up<C, TV, TD0, TS>(d, sK, omega, 0, ls, xcur);
 }
 
 template <int C, typename TV, typename TD0, typename TS>
@@ -628,29 +637,30 @@ EDGE_D void b_pcg_problem(const BatchDesc& d, const FineK<TV>& sK, const double*
   if (bb == 0.0) done = 1;  // nothing to solve: residual 0, like a converged solve
   if (*d.chol_status) done = 3;
   while (!done) {
-    const double rz_new = TM::sum(b_vcycle<C, TV, TD0, TS>(d, sK, omega, sb), sh, ph);
+    b_vcycle<C, TV, TD0, TS>(d, sK, omega, sb);
+    const double rz_new = b_dot<C>(nv, r, z, sh, ph);
     const double beta = iter == 0 ? 0.0 : rz_new / rz;
     for (long long k = TM::first(); k < nv; k += TM::stride())
       p[k] = iter == 0 ? (double)z[k] : (double)z[k] + beta * p[k];
     TM::sync();
-    double acc = 0.0;
-    b_fine2<C, double, double>(g, [&](long long s, int c) { return p[c * n + s]; }, d.E64, d.mask, sK64,
-                               [&](long long s, const double* own, const double* Au) {
-                                 for (int c = 0; c < 2; ++c) {
-                                   q[c * n + s] = Au[c];
-                                   acc += own[c] * Au[c];
-                                 }
-                               });
-    const double pq = TM::sum(acc, sh, ph);
+    const double pq = TeamSum<C>::run([&](int first, int step, double& acc) {
+      b_fine2<C, double, double>(g, [&](long long s, int c) { return p[c * n + s]; }, d.E64, d.mask, sK64,
+                                 [&](long long s, const double* own, const double* Au) {
+                                   for (int c = 0; c < 2; ++c) {
+                                     q[c * n + s] = Au[c];
+                                     acc += own[c] * Au[c];
+                                   }
+                                 }, first, step);
+    }, sh, ph);
     const double alpha = rz_new / pq;
-    double racc = 0.0;
-    for (long long k = TM::first(); k < nv; k += TM::stride()) {
-      x[k] = x[k] + alpha * p[k];
-      const double rv = r[k] - alpha * q[k];
-      r[k] = rv;
-      racc += rv * rv;
-    }
-    rr = TM::sum(racc, sh, ph);
+    rr = TeamSum<C>::run([&](int first, int step, double& acc) {
+      for (long long k = first; k < nv; k += step) {
+        x[k] = x[k] + alpha * p[k];
+        const double rv = r[k] - alpha * q[k];
+        r[k] = rv;
+        acc += rv * rv;
+      }
+    }, sh, ph);
     rz = rz_new;
     ++iter;
     const double R = sqrt(rr) / sqrt(bb);
@@ -725,7 +735,7 @@ template <typename TV, typename TD0, typename TS, int BT, int C>
 __global__ void __launch_bounds__(BT) k_batch_pcg(const BatchDesc* D, int nprob, unsigned* queue, double tol,
                                                   int maxiter, long long* tns) {
   using TM = Team<C>;
-  __shared__ double sh[33 + 2 * C];
+  __shared__ double sh[TeamSum<C>::SH];
   __shared__ double sb[BATCH_COARSE_SMEM];
   __shared__ TV sK[64];
   __shared__ double sK64[64];

@@ -355,7 +355,9 @@ int edge_batch_destroy(edge_batch* b);
  * thread block cluster of that many blocks solves each problem together).  Supported: team 1
  * with 256, 512 (default) or 1024 threads; team 2, 4 or 8 with 512 or 1024 threads.  With team > 1,
  * a batch small enough for all its solves to run at once gets a team size per problem instead (1 to
- * 16 blocks by its DOFs and previous iterations) when that is predicted to finish sooner. */
+ * 16 blocks by its DOFs and previous iterations) when that is predicted to finish sooner.  Team sizes
+ * change the time only: a problem's results are the same bits whatever team solves it and whatever is
+ * solved beside it (for one number of threads). */
 int edge_batch_set_threads(edge_batch* b, int threads, int team);
 /* With team > 1: problems with fewer than split_dof DOFs (default 0 = none) are solved
  * by single blocks of small_threads threads (256, 512 or 1024, the default) in a second

@@ -230,3 +230,31 @@ def test_large_coarsest_levels_stay_out_of_the_one_launch_cycle(precision):
         assert two - one == 2 * ns + 3
     three = _launches_per_iteration((64, 64), 3, 3, precision)       # 162 coarsest DOFs: one launch
     assert three < two
+
+
+@pytest.mark.parametrize("threads", [512, 1024])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batched_result_does_not_depend_on_the_company(precision, threads):
+    """Three SIMP iterations of the same problems, alone and in two companies, by teams of 1 to 16 blocks
+    (chosen per problem with team > 1; split_dof = 1 keeps the caller's team): the same bits, as every
+    step of a solve is node by node and its sums have one order.  Sizes from less than one to several
+    of a block's passes over the nodes."""
+    import torch
+    from edge_to_b200 import batch
+    specs = [batch.random_spec(i, seed=21, nelx_range=(nx, nx), nely_range=(ny, ny))
+             for i, (nx, ny) in enumerate([(24, 8), (60, 20), (64, 40), (120, 44), (200, 90), (300, 120)])]
+
+    def run(which, **kw):
+        b = batch.BatchSIMP([specs[i] for i in which], precision=precision, tol=1e-6, maxiter=400, persistent=True,
+                            block_threads=threads, **kw)
+        b.step(3)
+        return {i: (it["rho"].cpu(), it["dr"].cpu(), u.cpu(), it["comp"], it["pcg"])
+                for i, it, u in zip(which, b.items, b.batch.U)}
+    ref = run(range(6), team=1)
+    others = [run(range(6), team=4), run([5, 0, 2], team=8), run([1, 3, 4], team=2, split_dof=1)]
+    others += [run([i], team=4) for i in (0, 3, 5)]
+    for o in others:
+        for i, got in o.items():
+            for a, b in zip(got[:3], ref[i][:3]):
+                assert torch.equal(a, b), i
+            assert got[3:] == ref[i][3:], i
