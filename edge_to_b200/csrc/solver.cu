@@ -343,7 +343,7 @@ struct Prob {
   bool bd = false;
   int cur_cat = 0;
   std::vector<cudaEvent_t> bev;
-  std::vector<int> bcat;
+  std::vector<int> bcat, bcnt;  // category and number of launches of each event pair
   size_t bev_used = 0;
 
   template <typename T> T* alloc(size_t n) {
@@ -371,34 +371,42 @@ struct Prob {
 };
 
 
-// Every kernel launch of the solve path goes through here: counted for the benchmark's
-// launch tally and checked immediately.
-template <typename... KArgs, typename... Args>
-static void launch(Prob& P, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+// Every kernel launch of a problem goes through here: counted for the benchmark's launch tally, timed
+// under the current category while the breakdown is on, and checked immediately.  f() launches on
+// P.stream (its work is one sequence there) and returns how many kernels it launched.
+template <class F> static void launches(Prob& P, F&& f) {
   const bool rec = P.bd && P.bev_used + 2 <= P.bev.size();
   if (rec) CK(cudaEventRecord(P.bev[P.bev_used], P.stream));
-  if (P.pdl && P.capturing) {  // only on the library's own capture streams
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = P.stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
-  } else {
-    kern<<<grid, block, smem, P.stream>>>(static_cast<KArgs>(args)...);
-  }
-  ++P.nlaunch;
+  const int n = f();
+  P.nlaunch += n;
   KCHECK();
   if (rec) {
     CK(cudaEventRecord(P.bev[P.bev_used + 1], P.stream));
     P.bev_used += 2;
     P.bcat.push_back(P.cur_cat);
+    P.bcnt.push_back(n);
   }
+}
+template <typename... KArgs, typename... Args>
+static void launch(Prob& P, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  launches(P, [&] {
+    if (P.pdl && P.capturing) {  // only on the library's own capture streams
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = grid;
+      cfg.blockDim = block;
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = P.stream;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+    } else {
+      kern<<<grid, block, smem, P.stream>>>(static_cast<KArgs>(args)...);
+    }
+    return 1;
+  });
 }
 
 // Launch categories of the breakdown instrumentation.
@@ -1119,8 +1127,7 @@ static void mg_setup(Prob& P) {
   CK(cudaMemsetAsync(P.Adense, 0, (size_t)np * np * sizeof(double), P.stream));
   launch(P, k_st_to_dense<T>, cdiv(gL.n, 256), 256, 0, gL, (const T*)P.lv[L].S, P.Adense, np);
   CK(cudaMemsetAsync(P.chol_status, 0, sizeof(int), P.stream));
-  P.nlaunch += spd_inverse(P.Adense, nd, P.Ainv, P.inv_work, P.chol_status, P.stream);
-  KCHECK();
+  launches(P, [&] { return spd_inverse(P.Adense, nd, P.Ainv, P.inv_work, P.chol_status, P.stream); });
 }
 
 // ------------------------------------------------------------------ V-cycle
@@ -1178,16 +1185,11 @@ static void launch_tail(Prob& P, int l0) {
   cfg.stream = P.stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const bool rec = P.bd && P.bev_used + 2 <= P.bev.size();
-  if (rec) CK(cudaEventRecord(P.bev[P.bev_used], P.stream));
-  CK(cudaLaunchKernelEx(&cfg, k_vcycle_tail<TS>, T));
-  ++P.nlaunch;
-  KCHECK();
-  if (rec) {
-    CK(cudaEventRecord(P.bev[P.bev_used + 1], P.stream));
-    P.bev_used += 2;
-    P.bcat.push_back(CAT_STENCIL);
-  }
+  CatScope cat(P, CAT_STENCIL);
+  launches(P, [&] {
+    CK(cudaLaunchKernelEx(&cfg, k_vcycle_tail<TS>, T));
+    return 1;
+  });
 }
 
 static SolveKind solve_kind(bool mixed, bool bf16) {
@@ -1237,9 +1239,8 @@ static void fill_desc(const Prob& P, bool mixed, bool bf16, BatchDesc& d) {
   }
 }
 
-// Whether the V-cycle below the fine level runs as one cluster launch (2-D, no second visits; while
-// launches are timed one by one they stay separate).  The launch runs on eight SMs, so it has to be
-// small in two respects.  Level 1: a thread of the cluster for every node (64x32 elements, FP64: 96 us
+// Whether the V-cycle below the fine level runs as one cluster launch (2-D, no second visits).  The
+// launch runs on eight SMs, so it has to be small in two respects.  Level 1: a thread of the cluster for every node (64x32 elements, FP64: 96 us
 // per PCG iteration against 108 with separate launches, 160x96 128 / 139; 240x120 270 / 129).  The
 // coarsest DOFs, whose dense product grows with their square (FP64, three sweeps, us per iteration in
 // one launch / separate: 162 DOFs 93 / 105, 242 97 / 104, 306 80 / 79, 578 93 / 81, 1,250 195 / 84, 2,048
@@ -1248,8 +1249,7 @@ static void fill_desc(const Prob& P, bool mixed, bool bf16, BatchDesc& d) {
 // sweep in FP64 a level saves too few launches beyond 128 (128 DOFs 70.9 / 70.9, 200 59.4 / 57.5).  With one
 // coarse level there is nothing between the transfers to save (306 DOFs 40 / 36).
 static bool vtail2_usable(const Prob& P) {
-  if (P.dim != 2 || P.bd || P.prof || (P.cycle_w && !P.w_levels.empty()) || P.n_level < 2 || P.n_level >= BATCH_MAXL)
-    return false;
+  if (P.dim != 2 || (P.cycle_w && !P.w_levels.empty()) || P.n_level < 2 || P.n_level >= BATCH_MAXL) return false;
   const int nd_max = P.prec != EDGE_FP64 ? 320 : P.sweeps(1) >= 2 ? 240 : 128;
   return (long long)P.lv[1].g.nx * P.lv[1].g.ny <= VTAIL_C * VTAIL_BT && P.nd <= nd_max;
 }
@@ -1257,8 +1257,8 @@ template <typename TV> static void vtail2(Prob& P) {
   constexpr bool mixed = std::is_same<TV, float>::value;
   BatchDesc d;
   fill_desc(P, mixed, P.st_bf16, d);
-  P.nlaunch += vtail2_launch(solve_kind(mixed, P.st_bf16), d, &P.st->omega, P.stream);
-  KCHECK();
+  CatScope cat(P, CAT_STENCIL);
+  launches(P, [&] { return vtail2_launch(solve_kind(mixed, P.st_bf16), d, &P.st->omega, P.stream); });
 }
 
 // Result in `out`; b and out have type T.  With dot_dst, the last fine sweep also
@@ -2102,14 +2102,16 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
   SolveCounts sc;
   P.it_graph = capture_graph(P, [&](int& depth) {
     const long long a0 = P.nlaunch;
-    P.nlaunch += oc_launch(n, P.it_rho, P.it_dr, A, vol, vf, move, P.ocp, P.it_rho_new, P.part, P.ticket, P.oc,
-                           nullptr, P.stream);
-    KCHECK();
+    launches(P, [&] {
+      return oc_launch(n, P.it_rho, P.it_dr, A, vol, vf, move, P.ocp, P.it_rho_new, P.part, P.ticket, P.oc, nullptr,
+                       P.stream);
+    });
     {
       CatScope cat(P, CAT_SENS);
-      P.nlaunch += filter_forward(F.g, F.taps, F.tile(), F.N, P.it_rho_new,
-                                  FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, g}, P.stream);
-      KCHECK();
+      launches(P, [&] {
+        return filter_forward(F.g, F.taps, F.tile(), F.N, P.it_rho_new,
+                              FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, g}, P.stream);
+      });
     }
     n_fixed0 = P.nlaunch - a0;
     sc = capture_solve_into(P, tol, maxiter, false, depth);
@@ -2120,8 +2122,7 @@ static void capture_iteration(Prob& P, const edge_filter& F, double A, double vo
              (const double*)P.x64, P.part, P.ticket, P.scal + 2);
       launch(P, k_dk<double>, nbe, 256, 0, g, (const double*)P.x64, P.ei.k3, P.ei.k2, (const double*)P.dK0b,
              P.ei.wht ? 1 : 0, (double*)nullptr, (const double*)P.rho_f, P.gsens, penalty, void_);
-      P.nlaunch += filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, P.it_dr_new, P.stream);
-      KCHECK();
+      launches(P, [&] { return filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, P.it_dr_new, P.stream); });
     }
     n_fixed1 = P.nlaunch - c0;
   });
@@ -2783,12 +2784,19 @@ int edge_matvec(edge_problem* p, const double* u_dev, double* out_dev) {
   // switch off or a result over its own input, the solver's operator between two conversions
   if (P.n_springs == 0 && user_grid_ok(g) && (P.dim == 2 || (P.ei.wht && P.use_tma)) &&
       !overlap(u_dev, P.n_dof, out_dev, P.n_dof)) {
-    if (P.dim == 2)
-      P.nlaunch += product2_user(g, k2_dense(P), P.E64, P.mask, u_dev, out_dev, P.stream);
-    else
-      P.nlaunch += product3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.E64, P.mask, P.eflag16, P.mpz, u_dev,
-                                 out_dev, P.stream);
-    KCHECK();
+    CatScope cat(P, CAT_FINE);
+    const bool rec = P.prof && P.pev_used + 2 <= P.pev.size();
+    if (rec) CK(cudaEventRecord(P.pev[P.pev_used], P.stream));
+    launches(P, [&] {
+      if (P.dim == 2) return product2_user(g, k2_dense(P), P.E64, P.mask, u_dev, out_dev, P.stream);
+      return product3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.E64, P.mask, P.eflag16, P.mpz, u_dev, out_dev,
+                           P.stream);
+    });
+    if (rec) {
+      CK(cudaEventRecord(P.pev[P.pev_used + 1], P.stream));
+      P.pev_used += 2;
+      P.pbytes.push_back((double)P.n_dof * 2 * sizeof(double) + (double)P.n_el * sizeof(double));
+    }
     return EDGE_OK;
   }
   launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, u_dev, P.b64);
@@ -2855,10 +2863,10 @@ int edge_process_grad(edge_problem* p, const double* U_dev, double* dk_dev) {
   // straight from the user's vector, unless the element matrix lacks the box structure (3-D) or the
   // result lies over the input
   if (user_grid_ok(g) && (P.dim == 2 || P.ei.wht) && !overlap(U_dev, P.n_dof, dk_dev, P.n_el)) {
-    if (P.dim == 2)
-      P.nlaunch += energy2_user(g, k2_dense(P), P.ei.wht ? &P.ei.k2 : nullptr, U_dev, dk_dev, P.stream);
-    else
-      P.nlaunch += energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, U_dev, dk_dev, P.stream);
+    launches(P, [&] {
+      if (P.dim == 2) return energy2_user(g, k2_dense(P), P.ei.wht ? &P.ei.k2 : nullptr, U_dev, dk_dev, P.stream);
+      return energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, U_dev, dk_dev, P.stream);
+    });
   } else {
     launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, U_dev, P.b64);
     launch(P, k_dk<double>, cdiv(P.n_el, 256), 256, 0, g, P.b64, P.ei.k3, P.ei.k2, P.dK0b, P.ei.wht ? 1 : 0, dk_dev,
@@ -3150,6 +3158,7 @@ int edge_breakdown_begin(edge_problem* p, int max_launches) {
   }
   P.bev_used = 0;
   P.bcat.clear();
+  P.bcnt.clear();
   P.bd = true;
   API_END
 }
@@ -3169,7 +3178,7 @@ int edge_breakdown_end(edge_problem* p, double* ms_by_cat, int* n_by_cat, int n_
     const int c = P.bcat[i / 2];
     if (c < n_cat) {
       ms_by_cat[c] += t;
-      n_by_cat[c] += 1;
+      n_by_cat[c] += P.bcnt[i / 2];
     }
   }
   P.bd = false;
@@ -3325,8 +3334,9 @@ static void oc_run(Prob& P, long long n, const double* rho, const double* dr, do
                    double move, double* rho_new) {
   CatScope cat(P, CAT_OC);
   if (n != P.n_el) fail(EDGE_EINVAL, "OC vector length does not match the number of elements");
-  P.nlaunch += oc_launch(n, rho, dr, A, vol, vf, move, P.ocp, rho_new, P.part, P.ticket, P.oc, P.oc_h, P.stream);
-  KCHECK();
+  launches(P, [&] {
+    return oc_launch(n, rho, dr, A, vol, vf, move, P.ocp, rho_new, P.part, P.ticket, P.oc, P.oc_h, P.stream);
+  });
   CK(cudaStreamSynchronize(P.stream));
 }
 
@@ -3669,9 +3679,10 @@ int edge_simp_solve_and_process(edge_problem* p, edge_filter* f, const double* r
   double* rf = rho_f_dev ? rho_f_dev : P.rho_f;
   const unsigned nbe = cdiv(P.n_el, 256);
   // rho_f = H rho ; E = clip(rho_f^p, void, 1)
-  P.nlaunch += filter_forward(f->g, f->taps, f->tile(), f->N, rho_dev, FilterOut{rf, P.E64, P.E32, penalty, void_, g},
-                              P.stream);
-  KCHECK();
+  launches(P, [&] {
+    return filter_forward(f->g, f->taps, f->tile(), f->N, rho_dev, FilterOut{rf, P.E64, P.E32, penalty, void_, g},
+                          P.stream);
+  });
   P.has_rho = true;
   // U = K(E)^-1 f (warm start from U_dev)
   launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, f_dev, P.b64);
@@ -3688,7 +3699,7 @@ int edge_simp_solve_and_process(edge_problem* p, edge_filter* f, const double* r
   // dr = H^T (p clip(rho_f)^(p-1) dk)
   launch(P, k_dk<double>, nbe, 256, 0, g, P.x64, P.ei.k3, P.ei.k2, P.dK0b, P.ei.wht ? 1 : 0, nullptr, rf, P.gsens,
                                           penalty, void_);
-  P.nlaunch += filter_transpose(f->g, f->taps, f->tile(), f->N, P.gsens, dr_dev, P.stream);
+  launches(P, [&] { return filter_transpose(f->g, f->taps, f->tile(), f->N, P.gsens, dr_dev, P.stream); });
   launch(P, k_slots_to_user<double>, cdiv(g.n, 256), 256, 0, g, P.x64, U_dev);
   KCHECK();
   CK(cudaMemcpyAsync(P.scal_h + 2, P.scal + 2, sizeof(double), cudaMemcpyDeviceToHost, P.stream));
@@ -4018,8 +4029,8 @@ int edge_batch_oc_update(edge_batch* b, const double* const* rho, const double* 
   try {
     CK(cudaMemcpyAsync(B.d_oc, B.h_oc, n * sizeof(BatchOcDesc), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(B.queue, 0, sizeof(unsigned), s));
-    P0.nlaunch += oc_batch_launch(B.d_oc, n, B.queue, move, B.d_res, B.d_iters, s);
-    KCHECK();
+    CatScope cat(P0, CAT_OC);
+    launches(P0, [&] { return oc_batch_launch(B.d_oc, n, B.queue, move, B.d_res, B.d_iters, s); });
   } catch (...) {
     P0.stream = saved0;
     throw;
@@ -4124,9 +4135,10 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
       Geo gr = g;  // the real grid's extents in the problem's slot layout
       gr.nx = B.nxr[i];
       gr.ny = B.nyr[i];
-      P.nlaunch += filter_forward(F.g, F.taps, F.tile(), F.N, rho[i],
-                                  FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, gr}, P.stream);
-      KCHECK();
+      launches(P, [&] {
+        return filter_forward(F.g, F.taps, F.tile(), F.N, rho[i], FilterOut{P.rho_f, P.E64, P.E32, penalty, void_, gr},
+                              P.stream);
+      });
       P.has_rho = true;
       launch(P, k_user_to_slots_pad, cdiv(g.n, 256), 256, 0, g, B.nxr[i], B.nyr[i], f[i], P.b64);
       if (use_last)
@@ -4178,8 +4190,7 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
              (const double*)P.x64, P.part, P.ticket, P.scal + 2);
       launch(P, k_dk<double>, nbe, 256, 0, gr, (const double*)P.x64, P.ei.k3, P.ei.k2, (const double*)P.dK0b,
              P.ei.wht ? 1 : 0, (double*)nullptr, (const double*)P.rho_f, P.gsens, penalty, void_);
-      P.nlaunch += filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, dr[i], P.stream);
-      KCHECK();
+      launches(P, [&] { return filter_transpose(F.g, F.taps, F.tile(), F.N, P.gsens, dr[i], P.stream); });
       launch(P, k_slots_to_user_pad, cdiv(g.n, 256), 256, 0, g, B.nxr[i], B.nyr[i], (const double*)P.x64, U[i]);
     } catch (...) {
       P.stream = saved;

@@ -253,3 +253,49 @@ def test_persistent_batch_at_full_size():
         ca, cc = np.array(ia["comp"]), np.array(ic["comp"])
         assert np.max(np.abs(ca - cc) / np.abs(ca)) < 1e-9, sp["index"]
         assert float(ic["rho"].mean()) <= sp["vf"] * (1 + 1e-4)
+
+
+@pytest.mark.parametrize("nel,rmin", [((48, 24), 1.5), ((16, 8, 8), 1.5)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_breakdown_times_every_launch(nel, rmin, precision):
+    """Per-category times of one SIMP iteration, a product and the energies: every launch that the tally
+    counts is in a category, the OC update, the set-up with the coarsest inverse and the filter in
+    theirs; and a 2-D solve runs as it does otherwise, its cycle below the fine level one launch."""
+    import ctypes
+    import torch
+    import edge_to_b200 as eb
+    from edge_to_b200 import _lib
+    dim = len(nel)
+    p, k, _, f = _problem(nel, 3)
+    mesh = k.mesh if hasattr(k, "mesh") else None
+    st = lambda x: eb.auto_stiffness(x, 1.0, 0.3)  # noqa: E731
+    mesh = mesh or (eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D)(*nel, *map(float, nel), stiffness=st)
+    flt = (eb.CuStructuredFilter2D if dim == 2 else eb.CuStructuredFilter3D)(mesh, rmin)
+    sv = eb.CuMultiGrid(mesh, k, tol=1e-6, n_level=2, maxiter=300, precision=precision)
+    mat = eb.SingleMaterial(E=1.0, nu=0.3, void=1e-9, penalty=3.0, volume_fraction=0.4)
+    opt = eb.CuTopOpt(mesh, mat, k, sv, flt, max_iter=1, move=0.2, ch_tol=0, fun_tol=0, verbose=False)
+    opt.f = f.reshape(opt.f.shape)
+    rho = torch.full((mesh.n_elements,), 0.4, dtype=torch.float64, device="cuda")
+    _, dr, _ = opt.solve_and_process(rho, 0)
+
+    def tally():
+        n = ctypes.c_longlong()
+        _lib.call("edge_launch_count", k.handle, ctypes.byref(n))
+        return n.value
+    n0 = tally()
+    _lib.call("edge_breakdown_begin", k.handle, 60000)
+    rho = opt.update_design(rho, dr)
+    opt.solve_and_process(rho, 0)
+    its = sv.last_iters
+    k.dot(f.reshape(-1))
+    k.process_grad(f.reshape(-1))
+    ms, nn = (ctypes.c_double * 9)(), (ctypes.c_int * 9)()
+    _lib.call("edge_breakdown_end", k.handle, ms, nn, 9)
+    assert sum(nn) == tally() - n0
+    for c in (1, 2, 4, 5, 7, 8):
+        assert nn[c] > 0 and ms[c] > 0.0, c
+    assert nn[8] >= 3  # both filter passes and the sensitivities
+    if dim == 2:
+        assert nn[2] >= its and nn[3] == nn[6] == 0
+    else:
+        assert nn[3] > 0 and nn[6] >= its
