@@ -1273,20 +1273,30 @@ static int user3_chunk(long long tiles, int rows) {
   return best_ly;
 }
 
-bool user_grid_ok(const Geo& g) {
-  if (g.dim == 2) return (g.ny + 3) / 4 <= 65535;
-  return 3LL * g.nx * g.nz < (1LL << 31) && (g.nx + 14) / 15 <= 65535 && g.ny <= 65535;
+// Tiles of k_user3 along z and x and the rows it marches over: product tiles overlap by one element.
+struct User3Tiles {
+  long long tz, tx;
+  int rows;
+};
+static User3Tiles user3_tiles(const Geo& g, bool product) {
+  auto up = [](int n, int step) { return (long long)(n + step - 1) / step; };
+  if (product) return {up(g.nz, 15), up(g.nx, U3_NC - 1), g.ny};
+  return {up(g.nz - 1, 16), up(g.nx - 1, U3_NC), g.ny - 1};
+}
+
+bool user_grid_ok(const Geo& g, bool product) {
+  constexpr int MAX_YZ = 65535;  // grid dimensions y and z
+  if (g.dim == 2) return (g.ny + 3) / 4 <= MAX_YZ;
+  return 3LL * g.nx * g.nz < (1LL << 31) && user3_tiles(g, product).tx <= MAX_YZ && g.ny <= MAX_YZ;
 }
 
 template <bool PRODUCT, class K3>
 static int user3_launch(const Geo& g, const K3& K, const double* E, const uint8_t* mask, const uint8_t* eflag16, int mpz,
                         const double* u, double* out, cudaStream_t stream) {
-  const int step = PRODUCT ? 15 : 16, sx = PRODUCT ? U3_NC - 1 : U3_NC, nz = PRODUCT ? g.nz : g.nz - 1, nx = PRODUCT ? g.nx : g.nx - 1;
-  const int rows = PRODUCT ? g.ny : g.ny - 1;
-  const unsigned tz = (unsigned)((nz + step - 1) / step), tx = (unsigned)((nx + sx - 1) / sx);
-  const int ly = user3_chunk((long long)tz * tx, rows);
-  k_user3<PRODUCT, K3><<<dim3(tz, tx, (unsigned)((rows + ly - 1) / ly)), 32 * U3_BX, 0, stream>>>(g, K, E, mask, eflag16,
-                                                                                              mpz, ly, u, out);
+  const User3Tiles t = user3_tiles(g, PRODUCT);
+  const int ly = user3_chunk(t.tz * t.tx, t.rows);
+  const dim3 grid((unsigned)t.tz, (unsigned)t.tx, (unsigned)((t.rows + ly - 1) / ly));
+  k_user3<PRODUCT, K3><<<grid, 32 * U3_BX, 0, stream>>>(g, K, E, mask, eflag16, mpz, ly, u, out);
   return 1;
 }
 int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* E, const uint8_t* mask,

@@ -99,8 +99,8 @@ int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, con
                   const uint8_t* eflag16, int mpz, const double* u, double* out, cudaStream_t stream);
 int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* u, double* dk,
                  cudaStream_t stream);
-// Grids that the launches above take (their tile counts are grid dimensions).
-bool user_grid_ok(const Geo& g);
+// Grids that the products (or energies) above take: their tile counts are grid dimensions.
+bool user_grid_ok(const Geo& g, bool product);
 
 // ------------------------------------------------------------------ coarsest level
 // Inverse of a symmetric positive definite matrix.  A: np x np row-major, np = inv_padded(nd), the nd x nd

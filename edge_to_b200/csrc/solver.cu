@@ -2782,7 +2782,7 @@ int edge_matvec(edge_problem* p, const double* u_dev, double* out_dev) {
   const Geo& g = P.g0;
   // one launch on the user's vectors; with springs, an element matrix without the box structure, the TMA
   // switch off or a result over its own input, the solver's operator between two conversions
-  if (P.n_springs == 0 && user_grid_ok(g) && (P.dim == 2 || (P.ei.wht && P.use_tma)) &&
+  if (P.n_springs == 0 && user_grid_ok(g, true) && (P.dim == 2 || (P.ei.wht && P.use_tma)) &&
       !overlap(u_dev, P.n_dof, out_dev, P.n_dof)) {
     CatScope cat(P, CAT_FINE);
     const bool rec = P.prof && P.pev_used + 2 <= P.pev.size();
@@ -2862,7 +2862,7 @@ int edge_process_grad(edge_problem* p, const double* U_dev, double* dk_dev) {
   const Geo& g = P.g0;
   // straight from the user's vector, unless the element matrix lacks the box structure (3-D) or the
   // result lies over the input
-  if (user_grid_ok(g) && (P.dim == 2 || P.ei.wht) && !overlap(U_dev, P.n_dof, dk_dev, P.n_el)) {
+  if (user_grid_ok(g, false) && (P.dim == 2 || P.ei.wht) && !overlap(U_dev, P.n_dof, dk_dev, P.n_el)) {
     launches(P, [&] {
       if (P.dim == 2) return energy2_user(g, k2_dense(P), P.ei.wht ? &P.ei.k2 : nullptr, U_dev, dk_dev, P.stream);
       return energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, U_dev, dk_dev, P.stream);

@@ -258,3 +258,18 @@ def test_batched_result_does_not_depend_on_the_company(precision, threads):
             for a, b in zip(got[:3], ref[i][:3]):
                 assert torch.equal(a, b), i
             assert got[3:] == ref[i][3:], i
+
+
+@pytest.mark.parametrize("nelx", [458744, 458745, 524280, 524281])
+def test_product_and_energy_of_very_long_bars(nelx):
+    """One row of elements around the lengths at which the one-launch product (tiles of 7 node columns) and
+    energies (8 element columns) reach the limit of 65,535 tiles: beyond it the calls take the converting
+    path.  FP64 roundings of sums of at most 8 x 24 products of order 1."""
+    import torch
+    nel = (nelx, 1, 1)
+    mesh, k, cons, E, u = _problem(nel, 5)
+    k.set_constraints(cons)
+    ref, dk = _dense(mesh, nel, E, u, cons)
+    ut = torch.as_tensor(u, device="cuda")
+    np.testing.assert_allclose(k.dot(ut).cpu().numpy(), ref, rtol=0, atol=3e-14)
+    np.testing.assert_allclose(k.process_grad(ut).cpu().numpy(), dk, rtol=0, atol=1e-13)
