@@ -1255,24 +1255,6 @@ k_user3(const Geo g, const __grid_constant__ K3 K, const double* __restrict__ E,
   cp_wait<0>();
 }
 
-// Planes per block: the number of y-chunks that needs the fewest layers in all, counting the waves of
-// 2 x 148 resident blocks and one and a half layers of start-up per block.
-static int user3_chunk(long long tiles, int rows) {
-  long long best = -1;
-  int best_ly = rows;
-  for (int c = 1; c <= rows && c <= 4096; ++c) {
-    const int ly = (rows + c - 1) / c;
-    const long long blocks = tiles * ((rows + ly - 1) / ly);
-    const long long cost = ((blocks + 443) / 444) * (2LL * ly + 3);
-    if (best < 0 || cost < best) {
-      best = cost;
-      best_ly = ly;
-    }
-    if (tiles * c > 444LL * 64) break;
-  }
-  return best_ly;
-}
-
 // Tiles of k_user3 along z and x and the rows it marches over: product tiles overlap by one element.
 struct User3Tiles {
   long long tz, tx;
@@ -1284,6 +1266,30 @@ static User3Tiles user3_tiles(const Geo& g, bool product) {
   return {up(g.nz - 1, 16), up(g.nx - 1, U3_NC), g.ny - 1};
 }
 
+// Rows per block: the number of y-chunks that needs the fewest layers in all, counting the waves of
+// resident blocks (three per SM) and one and a half layers of start-up per block.  Up to 4,096 candidates:
+// a plan of the grid, made once with the
+// problem (made in every call, the energies of 8 x 4,000 x 8 elements took 18.8 us instead of 8.8).
+int user3_rows(const Geo& g, bool product) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const User3Tiles t = user3_tiles(g, product);
+  const long long tiles = t.tz * t.tx, wave = 3LL * sms;
+  long long best = -1;
+  int best_ly = t.rows;
+  for (int c = 1; c <= t.rows && c <= 4096; ++c) {
+    const int ly = (t.rows + c - 1) / c;
+    const long long blocks = tiles * ((t.rows + ly - 1) / ly);
+    const long long cost = ((blocks + wave - 1) / wave) * (2LL * ly + 3);
+    if (best < 0 || cost < best) {
+      best = cost;
+      best_ly = ly;
+    }
+    if (tiles * c > wave * 64) break;
+  }
+  return best_ly;
+}
+
 bool user_grid_ok(const Geo& g, bool product) {
   constexpr int MAX_YZ = 65535;  // grid dimensions y and z
   if (g.dim == 2) return (g.ny + 3) / 4 <= MAX_YZ;
@@ -1292,22 +1298,21 @@ bool user_grid_ok(const Geo& g, bool product) {
 
 template <bool PRODUCT, class K3>
 static int user3_launch(const Geo& g, const K3& K, const double* E, const uint8_t* mask, const uint8_t* eflag16, int mpz,
-                        const double* u, double* out, cudaStream_t stream) {
+                        int ly, const double* u, double* out, cudaStream_t stream) {
   const User3Tiles t = user3_tiles(g, PRODUCT);
-  const int ly = user3_chunk(t.tz * t.tx, t.rows);
   const dim3 grid((unsigned)t.tz, (unsigned)t.tx, (unsigned)((t.rows + ly - 1) / ly));
   k_user3<PRODUCT, K3><<<grid, 32 * U3_BX, 0, stream>>>(g, K, E, mask, eflag16, mpz, ly, u, out);
   return 1;
 }
 int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* E, const uint8_t* mask,
-                  const uint8_t* eflag16, int mpz, const double* u, double* out, cudaStream_t stream) {
-  if (cube) return user3_launch<true>(g, *cube, E, mask, eflag16, mpz, u, out, stream);
-  return user3_launch<true>(g, K, E, mask, eflag16, mpz, u, out, stream);
+                  const uint8_t* eflag16, int mpz, int ly, const double* u, double* out, cudaStream_t stream) {
+  if (cube) return user3_launch<true>(g, *cube, E, mask, eflag16, mpz, ly, u, out, stream);
+  return user3_launch<true>(g, K, E, mask, eflag16, mpz, ly, u, out, stream);
 }
-int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* u, double* dk,
+int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, int ly, const double* u, double* dk,
                  cudaStream_t stream) {
-  if (cube) return user3_launch<false>(g, *cube, nullptr, nullptr, nullptr, 0, u, dk, stream);
-  return user3_launch<false>(g, K, nullptr, nullptr, nullptr, 0, u, dk, stream);
+  if (cube) return user3_launch<false>(g, *cube, nullptr, nullptr, nullptr, 0, ly, u, dk, stream);
+  return user3_launch<false>(g, K, nullptr, nullptr, nullptr, 0, ly, u, dk, stream);
 }
 
 // ------------------------------------------------------------------ coarsest level

@@ -91,14 +91,15 @@ int energy2_user(const Geo& g, const K2Dense& K, const KHat2<double>* box, const
                  cudaStream_t stream);
 
 // The same in 3-D, for element matrices with the box structure (KHat3, element_op.cuh) and, when
-// `cube` is given, its block form (equal edges, isotropic material: KCube64).
+// `cube` is given, its block form (equal edges, isotropic material: KCube64).  ly: user3_rows of the grid.
 struct KCube64 {
   double nd, no, sh, bd, bo, td, to, h7;  // nd and td without the shared part no / to
 };
 int product3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* E, const uint8_t* mask,
-                  const uint8_t* eflag16, int mpz, const double* u, double* out, cudaStream_t stream);
-int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, const double* u, double* dk,
+                  const uint8_t* eflag16, int mpz, int ly, const double* u, double* out, cudaStream_t stream);
+int energy3_user(const Geo& g, const KHat3<double>& K, const KCube64* cube, int ly, const double* u, double* dk,
                  cudaStream_t stream);
+int user3_rows(const Geo& g, bool product);
 // Grids that the products (or energies) above take: their tile counts are grid dimensions.
 bool user_grid_ok(const Geo& g, bool product);
 

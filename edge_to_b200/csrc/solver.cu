@@ -225,6 +225,7 @@ struct Prob {
   KCube kcube;             // block form of the same operator (cube elements)
   bool cube = false;       // kcube reproduces every entry of the transformed operator
   KCube64 kcube64;         // the same in FP64
+  int user_rows[2] = {0, 0};  // 3-D: rows per block of the one-launch product and energies
   bool cube64 = false;     // ... to FP64 rounding
   int blocks_per_sm = 4;   // y-chunking target of the fine kernel
   // per kind of fused cube launch (0: first sweep + residual, 1: last sweep + correction,
@@ -2280,6 +2281,7 @@ int edge_problem_create(int dim, const int* nel, const double* K0, int precision
     if (dim == 3) {
       P.k3p = pack3(P.ei.k3);
       P.cube = P.ei.wht && cube_form(P.ei.k3, P.kcube, P.kcube64, P.cube64);
+      for (int k = 0; k < 2; ++k) P.user_rows[k] = user3_rows(P.g0, k == 0);
     }
     const int nk = P.ei.nk;
     P.dK0b = P.alloc<double>(nk * nk);
@@ -2789,8 +2791,8 @@ int edge_matvec(edge_problem* p, const double* u_dev, double* out_dev) {
     if (rec) CK(cudaEventRecord(P.pev[P.pev_used], P.stream));
     launches(P, [&] {
       if (P.dim == 2) return product2_user(g, k2_dense(P), P.E64, P.mask, u_dev, out_dev, P.stream);
-      return product3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.E64, P.mask, P.eflag16, P.mpz, u_dev, out_dev,
-                           P.stream);
+      return product3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.E64, P.mask, P.eflag16, P.mpz, P.user_rows[0], u_dev,
+                           out_dev, P.stream);
     });
     if (rec) {
       CK(cudaEventRecord(P.pev[P.pev_used + 1], P.stream));
@@ -2865,7 +2867,7 @@ int edge_process_grad(edge_problem* p, const double* U_dev, double* dk_dev) {
   if (user_grid_ok(g, false) && (P.dim == 2 || P.ei.wht) && !overlap(U_dev, P.n_dof, dk_dev, P.n_el)) {
     launches(P, [&] {
       if (P.dim == 2) return energy2_user(g, k2_dense(P), P.ei.wht ? &P.ei.k2 : nullptr, U_dev, dk_dev, P.stream);
-      return energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, U_dev, dk_dev, P.stream);
+      return energy3_user(g, P.ei.k3, P.cube64 ? &P.kcube64 : nullptr, P.user_rows[1], U_dev, dk_dev, P.stream);
     });
   } else {
     launch(P, k_user_to_slots<double>, cdiv(g.n, 256), 256, 0, g, U_dev, P.b64);

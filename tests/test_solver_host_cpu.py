@@ -43,3 +43,18 @@ def test_sweep_choice_falls_back_when_no_contender_converges_again():
     best = pick_sweep_pattern(runs, _retime({(1, 1, 1): 100.0, (2, 2, 2): 60.0}, fail={(1, 1, 1), (2, 2, 2)}), m,
                               fallback=fallback)
     assert best == (0.0, [3, 3, 3], 0)
+
+
+def test_row_plan_of_the_one_launch_product_is_made_with_the_problem():
+    """The search for the rows per block tries up to 4,096 splits on the host: it runs at a problem's
+    creation, and the launch itself holds no loop."""
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "edge_to_b200", "csrc")
+    solver, fields = (open(os.path.join(csrc, f)).read() for f in ("solver.cu", "fields.cu"))
+    calls = [m.start() for m in re.finditer(r"user3_rows\(", solver)]
+    create = solver.index("\nint edge_problem_create(")
+    assert len(calls) == 1 and create < calls[0] < solver.index("\n}\n", create)
+    launch = fields[fields.index("static int user3_launch("):]
+    launch = launch[:launch.index("\n}\n")]
+    assert "<<<" in launch and "for (" not in launch and "user3_rows" not in launch and "user3_chunk" not in launch
