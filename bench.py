@@ -649,7 +649,7 @@ def run_tiles(args, cfg_name):
         _lib.call("edge_set_stencil_pair", h, 200000)
         _lib.call("edge_set_stencil_tiled", h, 200000)
         levels.append(row)
-    _lib.call("edge_set_stencil_quad", h, 20000)
+    _lib.call("edge_set_stencil_quad", h, 40000 if args.precision == "mixed" else 24000)
     return {"mode": "tiles", "workload": cfg_name, "precision": args.precision, "peak_GBps": peak,
             "peak_source": kind, "plain_bytes": plain_bytes, "sweep_bytes": sweep_bytes, "tiles": rows,
             "stencil_levels": levels}

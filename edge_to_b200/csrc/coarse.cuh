@@ -434,9 +434,12 @@ k_st3_apply2t(const Geo g, const float* __restrict__ u, const unsigned* __restri
 // For levels that leave the GPU waiting on latency: a Jacobi sweep of 225, 1,377 and 9,537 nodes takes
 // 4.6, 5.2 and 6.2 us in FP64 (4.1, 4.1 and 6.2 in FP32 on BF16 coefficients) against 10.3 with one
 // thread per node (26 dependent trips) and 9.5 with the four lanes per node it replaces.  Its warps read
-// every coefficient twice through L2, so larger levels keep one thread per node: 38,425 nodes 14.4
-// (FP64) and 10.3 (FP32) against 12.3 and 11.5, 70,785 nodes 27 and 16 against 18 and 12.
+// every coefficient twice through L2, so larger levels keep one thread per node, from where that is as
+// fast: a sweep of 23,548 slots takes 10.2 us against 10.4 and of 34,336 slots 12.3 against 10.6 in FP64;
+// in FP32 23,548 slots 8.2 / 10.3, 39,072 slots 10.3 / 11.1, 54,612 slots 12.3 / 12.3, 66,420 slots 14.3 /
+// 12.3 on BF16 coefficients, and within 1 us of these on FP32 ones.
 constexpr int ST3D_WARPS = 14;
+constexpr long long ST3D_MAX_FP64 = 24000, ST3D_MAX_MIXED = 40000;  // slots
 template <typename T, typename TS, class Epi>
 __global__ void __launch_bounds__(32 * ST3D_WARPS)
 k_st3_apply_d(const Geo g, const T* __restrict__ u, const TS* __restrict__ S, Epi epi, double* part, unsigned* ticket,

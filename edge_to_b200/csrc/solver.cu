@@ -234,7 +234,11 @@ struct Prob {
   int kind_variant[3] = {-1, -1, -1};
   int kind_bps[3] = {0, 0, 0};
   bool kind_tune = true;  // edge_autotune_fine also picks the per-kind tiles
-  long long st_quad_max = 20000;   // 3-D stencil levels with at most this many slots use k_st3_apply_d
+  // 3-D stencil levels with at most this many slots use k_st3_apply_d (below zero: by precision)
+  long long st_quad_max = -1;
+  long long quad_max() const {
+    return st_quad_max >= 0 ? st_quad_max : prec == EDGE_FP64 ? ST3D_MAX_FP64 : ST3D_MAX_MIXED;
+  }
   bool st_bf16 = true;             // mixed precision: apply the coarse stencils from BF16 copies
   // mixed precision: the residual recurrence between FP64 replacements is stored in FP32
   // (arithmetic and r.r in FP64); false keeps an FP64 recurrence with an FP32 copy
@@ -961,7 +965,7 @@ static void fine_apply_dense(Prob& P, const T* u, Epi epi, double* dot_dst) {
 template <typename T, class Epi, typename TS = T>
 static void st_apply(Prob& P, const Geo& g, const T* u, const TS* S, Epi epi, double* dot_dst) {
   CatScope cat(P, CAT_STENCIL);
-  if (g.dim == 3 && g.n <= P.st_quad_max)
+  if (g.dim == 3 && g.n <= P.quad_max())
     launch(P, k_st3_apply_d<T, TS, Epi>, dim3(cdiv(g.n, 32)), dim3(32 * ST3D_WARPS), 0, g, u, S, epi, P.part, P.ticket,
            dot_dst);
   else if (g.dim == 3 && P.st_pair && std::is_same<T, float>::value && g.n >= P.st_pair_min)
@@ -981,7 +985,7 @@ static void level_apply(Prob& P, int l, const T* u, Epi epi, double* dot_dst = n
   }
   if constexpr (std::is_same<T, float>::value) {
     if (P.st_bf16 && P.st_pair && P.lv[l].S16t && P.st_tile_min >= 0 && P.lv[l].g.n >= P.st_tile_min &&
-        P.lv[l].g.n > P.st_quad_max) {
+        P.lv[l].g.n > P.quad_max()) {
       CatScope cat(P, CAT_STENCIL);
       const Geo& g = P.lv[l].g;
       launch(P, k_st3_apply2t<Epi>, dim3(cdiv(g.n / 2, 128)), dim3(128), 0, g, u, (const unsigned*)P.lv[l].S16t, epi,
@@ -1810,7 +1814,7 @@ static void mg_setup_prec(Prob& P) {
 static std::vector<double> graph_key(const Prob& P, double tol, int maxiter, bool cg = false) {
   std::vector<double> k = {cg ? -1.0 : (double)P.prec, tol, (double)maxiter, (double)P.n_level, (double)P.n_smooth, P.omega,
                            P.min_omega, (double)P.cycle_w, (double)P.tile_variant, (double)P.blocks_per_sm,
-                           (double)P.st_quad_max, (double)P.n_springs, (double)P.use_tma, (double)P.has_cons,
+                           (double)P.quad_max(), (double)P.n_springs, (double)P.use_tma, (double)P.has_cons,
                            (double)P.st_bf16, (double)P.st_pair, (double)P.st_pair_min, (double)P.st_tile_min,
                            (double)P.gal_axis, (double)P.res32,
                            (double)P.pdl, (double)P.fuse, (double)P.tail_l0, (double)P.omega_carry, (double)(P.omega_carry && P.omega_started),

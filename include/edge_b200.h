@@ -182,8 +182,8 @@ int edge_set_residual32(edge_problem* p, int enable);
  * Host-driven solves always use plain order. */
 int edge_set_pdl(edge_problem* p, int enable);
 /* Coarse 3-D levels with at most max_slots slots use the warp-per-direction stencil kernel
- * (latency-bound small levels); larger levels one thread per node.  Default 20000 (at 38k nodes
- * one thread per node is already as fast). */
+ * (latency-bound small levels); larger levels one thread per node.  Default 24000 in FP64 and
+ * 40000 in mixed precision (where one thread per node becomes as fast). */
 int edge_set_stencil_quad(edge_problem* p, long long max_slots);
 /* Benchmark helper: average device time (ms) of `reps` Jacobi sweeps of the stencil operator
  * on coarse level 1 <= level < n_level, in the problem's precision (hierarchy built). */

@@ -273,3 +273,28 @@ def test_product_and_energy_of_very_long_bars(nelx):
     ut = torch.as_tensor(u, device="cuda")
     np.testing.assert_allclose(k.dot(ut).cpu().numpy(), ref, rtol=0, atol=3e-14)
     np.testing.assert_allclose(k.process_grad(ut).cpu().numpy(), dk, rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_default_kernel_of_a_medium_stencil_level(precision):
+    """Level 1 of 34,848 slots: one thread per node in FP64 (10.6 us a sweep against 12.3), a warp per
+    direction in mixed precision (8.5 against 10.3).  The two add a node's terms in different orders, so
+    the bits of a solve tell which one the default took."""
+    import torch
+    import edge_to_b200 as eb
+    from edge_to_b200 import _lib
+    nel = (64, 64, 56)
+    mesh, k, _, E, _ = _problem(nel, 2)
+    k.set_constraints(np.arange(3 * 65 * 57))
+    f = np.zeros(k.shape[0])
+    f[-1] = -1.0
+    f = torch.as_tensor(f, device="cuda")
+    got = []
+    for quad in (None, 20000, 60000):
+        sv = eb.CuMultiGrid(mesh, k, tol=1e-300, n_level=3, maxiter=3, precision=precision, autotune=False,
+                            tune_sweeps=False)
+        if quad is not None:
+            _lib.call("edge_set_stencil_quad", k.handle, quad)
+        got.append(sv.solve(f, torch.as_tensor(E, device="cuda"), use_last=False)[0].cpu())
+    assert not torch.equal(got[1], got[2])
+    assert torch.equal(got[0], got[1 if precision == "fp64" else 2])
