@@ -512,16 +512,18 @@ int oc_launch(long long n, const double* rho, const double* dr, double A, double
   cfg.stream = stream;
   cfg.attrs = at;
   if (n <= OC_CLUSTER_MAX) {
-    // on every call: the attribute belongs to the current device's context, not to the process
-    if (cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = OC_TEAM;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(OC_TEAM);
     cfg.blockDim = dim3(OC_TEAM_THREADS);
-    cudaLaunchKernelEx(&cfg, k_oc_cluster, BatchOcDesc{n, rho, dr, ocp, rho_new, A, vol, vf}, move, st, host);
-    return 1;
+    // the attribute on every call: it belongs to the current device's context, not to the process
+    if (cudaFuncSetAttribute(k_oc_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaLaunchKernelEx(&cfg, k_oc_cluster, BatchOcDesc{n, rho, dr, ocp, rho_new, A, vol, vf}, move, st, host) ==
+            cudaSuccess)
+      return 1;
+    cudaGetLastError();  // 16 blocks do not fit side by side (a part of a GPU): the grid's passes take any size
   }
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
