@@ -540,7 +540,9 @@ int oc_launch(long long n, const double* rho, const double* dr, double A, double
 
 int oc_batch_launch(const BatchOcDesc* D, int nprob, unsigned* queue, double move, double* lam_out, int* steps_out,
                     cudaStream_t stream) {
-  k_oc_batch<<<std::max(1, std::min(nprob, 148)), OCB_THREADS, 0, stream>>>(D, nprob, queue, move, lam_out, steps_out);
+  int dev = 0, sms = 1;  // 128 registers a thread: one block per SM
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  k_oc_batch<<<std::max(1, std::min(nprob, sms)), OCB_THREADS, 0, stream>>>(D, nprob, queue, move, lam_out, steps_out);
   return 1;
 }
 

@@ -4085,11 +4085,11 @@ int edge_batch_solve_and_process(edge_batch* b, const double* const* rho, double
   int n_large = n;
   double w_large = 0.0, w_small = 0.0;
   B.sized.clear();
-  if (B.team > 1 && B.split_dof == 0 && n <= 148) {
-    int clusters = 0, dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    clusters = batch_clusters16(solve_kind(mixed, bf16), B.threads);
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (B.team > 1 && B.split_dof == 0 && n <= sms) {
+    const int clusters = batch_clusters16(solve_kind(mixed, bf16), B.threads);
     std::vector<int> size;
     const double t = batch_sizes(B, std::min(16 * clusters, sms), size);
     if (t > 0.0 && t < batch_queue_time(B, sms)) {  // queue positions by size, then by cost
