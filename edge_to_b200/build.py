@@ -15,7 +15,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libedge_b200.so")
 OBJDIR = os.path.join(HERE, "_build")
-SOURCES = ["solver.cu", "batch.cu", "fields.cu"]
+SOURCES = ["solver.cu", "batch.cu", "vtail.cu", "fields.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -1,4 +1,4 @@
-// The batched solve and the one-launch 2-D V-cycle tail (batch.cu): descriptors and launchers.
+// The batched solve (batch.cu) and the one-launch 2-D V-cycle tail (vtail.cu): descriptors and launchers.
 #pragma once
 #include "common.cuh"
 #include "element_op.cuh"

@@ -1200,7 +1200,7 @@ static void launch_tail(Prob& P, int l0) {
 static SolveKind solve_kind(bool mixed, bool bf16) {
   return !mixed ? SOLVE_FP64 : bf16 ? SOLVE_MIXED_BF16 : SOLVE_MIXED_FP32;
 }
-// The descriptor of a 2-D problem for the kernels of batch.cu.
+// The descriptor of a 2-D problem for the kernels of batch.cu and vtail.cu.
 static void fill_desc(const Prob& P, bool mixed, bool bf16, BatchDesc& d) {
   std::memset(&d, 0, sizeof(d));
   d.n_level = P.n_level;

@@ -25,19 +25,18 @@ def body(src, name):
 def test_peer_shared_memory_is_addressed_behind_a_cluster_barrier():
     """A block of a cluster may be addressed through map_shared_rank only once it has started, which a
     cluster barrier establishes: every use in a kernel comes after one."""
-    users = {f for f in os.listdir(CSRC) if "map_shared_rank" in source(f)}
-    assert users == {"fields.cu", "batch.cu"}
+    uses = {f: source(f).count("map_shared_rank") for f in os.listdir(CSRC)}
+    assert {f: n for f, n in uses.items() if n} == {"fields.cu": 1, "batch_ops.cuh": 1, "batch.cu": 1}
     oc = body(source("fields.cu"), "oc_team")
-    assert source("fields.cu").count("map_shared_rank") == oc.count("map_shared_rank") == 1
+    assert oc.count("map_shared_rank") == 1
     first = re.search(r"barrier_wait\(\)|this_cluster\(\)\.sync\(\)", oc)
     assert first and first.start() < oc.index("map_shared_rank") < oc.index("team_sum(v)")
     # the batched solve: the queue's barrier comes before the first read of a peer and before the solve,
-    # whose sums (Team::sum) write to peers
-    src = source("batch.cu")
-    kern = body(src, "k_batch_pcg")
-    assert src.count("map_shared_rank") == 2 and kern.count("map_shared_rank") == 1
+    # whose sums (TeamSum::run) write to peers; the one-launch cycle sums nothing
+    kern = body(source("batch.cu"), "k_batch_pcg")
+    assert kern.count("map_shared_rank") == 1
     assert kern.index("TM::sync()") < kern.index("map_shared_rank") < kern.index("b_pcg_problem")
-    assert "::sum(" not in body(src, "k_vtail2")
+    assert "TeamSum" not in source("vtail.cu")
 
 
 def test_stencil_warps_meet_at_one_barrier():

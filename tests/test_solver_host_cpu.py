@@ -58,3 +58,15 @@ def test_row_plan_of_the_one_launch_product_is_made_with_the_problem():
     launch = fields[fields.index("static int user3_launch("):]
     launch = launch[:launch.index("\n}\n")]
     assert "<<<" in launch and "for (" not in launch and "user3_rows" not in launch and "user3_chunk" not in launch
+
+
+def test_the_one_launch_cycle_is_loaded_without_the_batched_solve():
+    """A process loads all kernels of a translation unit at its first launch from it: the one-launch 2-D
+    cycle, which every small 2-D solve uses, stays apart from the 33 kernels of the batched solve (60 ms
+    of a process's first solve)."""
+    import os
+    from edge_to_b200 import build
+    units = {s: open(os.path.join(build.CSRC, s)).read() for s in build.SOURCES}
+    cycle = [s for s, t in units.items() if "k_vtail2<" in t]
+    batch = [s for s, t in units.items() if "k_batch_pcg<" in t]
+    assert len(cycle) == len(batch) == 1 and cycle != batch
