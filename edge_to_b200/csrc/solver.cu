@@ -3796,21 +3796,27 @@ __global__ void k_batch_gather(const BatchDesc* D, const double* const* scal, in
 // Team sizes of a batch whose problems all fit on the GPU at once.  With teams of one size such a batch
 // takes as long as its costliest problem while SMs stay idle (24 problems of 10k-220k DOFs on teams
 // of four: 285 ms, the mean problem 90).  A problem's solve takes about its iterations times
-// (I_c + DOFs / c) on c blocks (fitted to 24 problems at c = 1, 4 and 8: a step of a team costs a
-// barrier and two trips to L2 whatever the size; a single block's barrier is nearly free), so the
-// smallest time T is sought for which the smallest sizes with time <= T fit.  Sizes are powers of two
-// up to 16 and their sum stays within the blocks that clusters of 16 could fill: powers of two then
-// pack into the GPCs.  24 problems: 285 -> 160 ms (every SM busy, problems end between 92 and 160 ms;
-// 137 with the marching fine operator).  Returns the sizes by queue position
-// and the predicted time of that choice.
+// (I_c + DOFs / c) on c blocks (batch_time), so the smallest time T is sought for which the smallest
+// sizes with time <= T fit.  Sizes are powers of two up to 16 and their sum stays within the blocks that
+// clusters of 16 could fill: powers of two then pack into the GPCs.  24 problems: 285 -> 160 ms (every SM
+// busy, problems end between 92 and 160 ms; 137 with the marching fine operator).  Returns the sizes by
+// queue position and the predicted time of that choice.
+//
+// I_c, in DOFs, fitted to the solves of 48 problems of 10k-220k DOFs by teams of 1, 2, 4 and 8 blocks of
+// 1,024 threads (residuals 3-8 %): mixed 1,917, 4,954, 5,972, 5,996 at 9-11 ns a DOF, FP64 2,870, 5,346,
+// 6,888, 6,821 at 12-14 ns: a step of a team costs a barrier and two trips to L2 whatever the size, a
+// single block's barrier less.
+static double batch_time(const edge_batch& B, int problem, int c) {
+  const Prob& P = B.probs[problem]->P;
+  const double dof = (double)std::max<long long>(1, P.n_dof);
+  const double its = std::max(1.0, (double)B.cost[problem] / dof);
+  const double one = P.prec == EDGE_FP64 ? 2900.0 : 1900.0, more = P.prec == EDGE_FP64 ? 6800.0 : 5900.0;
+  return its * ((c == 1 ? one : more) + dof / c);
+}
 static double batch_sizes(const edge_batch& B, int budget, std::vector<int>& size) {
   static const int SZ[5] = {1, 2, 4, 8, 16};
   const int n = (int)B.order.size();
-  auto time = [&](int k, int c) {
-    const double dof = (double)std::max<long long>(1, B.probs[B.order[k]]->P.n_dof);
-    const double its = std::max(1.0, (double)B.cost[B.order[k]] / dof);
-    return its * ((c == 1 ? 500.0 : 5800.0) + dof / c);
-  };
+  auto time = [&](int k, int c) { return batch_time(B, B.order[k], c); };
   std::vector<double> ts;
   for (int k = 0; k < n; ++k)
     for (int c : SZ) ts.push_back(time(k, c));
@@ -3845,8 +3851,7 @@ static double batch_sizes(const edge_batch& B, int budget, std::vector<int>& siz
 static double batch_queue_time(const edge_batch& B, int sms) {
   double most = 0.0, sum = 0.0;
   for (int i : B.order) {
-    const double dof = (double)std::max<long long>(1, B.probs[i]->P.n_dof);
-    const double t = std::max(1.0, (double)B.cost[i] / dof) * ((B.team == 1 ? 500.0 : 5800.0) + dof / B.team);
+    const double t = batch_time(B, i, B.team);
     most = std::max(most, t);
     sum += t;
   }
