@@ -298,3 +298,62 @@ def test_default_kernel_of_a_medium_stencil_level(precision):
         got.append(sv.solve(f, torch.as_tensor(E, device="cuda"), use_last=False)[0].cpu())
     assert not torch.equal(got[1], got[2])
     assert torch.equal(got[0], got[1 if precision == "fp64" else 2])
+
+
+@pytest.mark.parametrize("nel,n_level", [((16, 14), 1), ((62, 62), 1), ((64, 32), 2), ((10, 8, 8), 1), ((16, 8, 8), 2)])
+def test_coarsest_inverse_with_void_elements(nel, n_level):
+    """A block of void elements (1e-9) in a solid grid: the pivots of the block sweeps span the contrast.
+    The PCG takes the oracle's iterations; the solutions then differ by roundings of the contrast at most
+    (1e9 machine roundings of the largest displacement, 1e-6)."""
+    import torch
+    import edge_to_b200 as eb
+    dim = len(nel)
+    p = (topopt.mbb_problem if dim == 2 else topopt.cantilever_problem)(
+        *nel, vf=0.4, mg_kwargs=dict(tol=1e-8, n_level=n_level, maxiter=1000, variant="gpu"))
+    E = np.ones(nel)
+    E[tuple(slice(n // 4, n // 2) for n in nel)] = 1e-9
+    E = E.ravel()
+    ref, _ = p.solver.solve(ops.assemble(p.grid, p.K0, E, p.cons), p.f, use_last=False)
+    mesh = (eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D)(
+        *nel, *map(float, nel), stiffness=lambda x: eb.auto_stiffness(x, 1.0, 0.3))
+    k = eb.CuStructuredStiffnessKernel(mesh)
+    k.add_constraints(p.cons)
+    sv = eb.CuMultiGrid(mesh, k, tol=1e-8, n_level=n_level, maxiter=1000)
+    x, res = sv.solve(torch.as_tensor(p.f, device="cuda"), torch.as_tensor(E, device="cuda"), use_last=False)
+    assert res < 1e-8 and sv.last_iters == p.solver.pcg_iters[-1]
+    np.testing.assert_allclose(x.cpu().numpy(), ref, rtol=0, atol=1e-6 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("nel", [(40, 37), (9, 20, 33)])
+@pytest.mark.parametrize("rmin", [1.0, 1.5, 2.0, 2.9])
+def test_filter_keeps_an_infinity_to_its_taps(nel, rmin):
+    """An infinite value reaches exactly the elements that have a tap on it: a tap that the stencil does
+    not have is not a product with zero.  The others as in the finite test."""
+    import torch
+    import edge_to_b200 as eb
+    dim = len(nel)
+    mesh = (eb.CuStructuredMesh2D if dim == 2 else eb.CuStructuredMesh3D)(*nel, *map(float, nel))
+    flt = (eb.CuStructuredFilter2D if dim == 2 else eb.CuStructuredFilter3D)(mesh, rmin)
+    x = np.random.default_rng(3).uniform(size=nel)
+    x[tuple(n // 2 for n in nel)] = np.inf
+    x[tuple(0 for _ in nel)] = np.inf
+    offs, w = flt.offsets.cpu().numpy(), flt.weights.cpu().numpy()
+    idx = np.stack(np.meshgrid(*[np.arange(n) for n in nel], indexing="ij"), -1)
+    num, norm = np.zeros(nel), np.zeros(nel)
+    for o, wk in zip(offs, w):
+        nb = idx + o
+        ok = np.all((nb >= 0) & (nb < np.array(nel)), axis=-1)
+        num[ok] += wk * x[tuple(nb[ok].T)]
+        norm[ok] += wk
+    trans = np.zeros(nel)
+    for o, wk in zip(offs, w):
+        nb = idx + o
+        ok = np.all((nb >= 0) & (nb < np.array(nel)), axis=-1)
+        trans[ok] += wk / norm[tuple(nb[ok].T)] * x[tuple(nb[ok].T)]
+    xt = torch.as_tensor(x.ravel(), device="cuda")
+    for got, ref, atol in ((flt.dot(xt), num / norm, 2e-15), (flt.T.dot(xt), trans, 2e-14)):
+        got, ref = got.cpu().numpy(), ref.ravel()
+        np.testing.assert_array_equal(np.isinf(got), np.isinf(ref))
+        assert not np.isnan(got).any()
+        f = np.isfinite(ref)
+        np.testing.assert_allclose(got[f], ref[f], rtol=0, atol=atol)
