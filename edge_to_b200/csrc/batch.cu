@@ -139,6 +139,9 @@ EDGE_D long long global_ns() {
 
 // tns (may be null): start and end of each problem's solve (global timer, ns), for the
 // benchmark's load-balance record.
+//
+// The 1,024-thread forms sit at the limit of 64 registers and spill (teams of 4, bytes stored / loaded:
+// mixed 1,992 / 3,188, FP64 5,168 / 8,060); the 512-thread forms have 128 and spill 12 to 40 bytes.
 template <typename TV, typename TD0, typename TS, int BT, int C>
 __global__ void __launch_bounds__(BT) k_batch_pcg(const BatchDesc* D, int nprob, unsigned* queue, double tol,
                                                   int maxiter, long long* tns) {

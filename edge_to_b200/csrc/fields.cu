@@ -497,11 +497,11 @@ k_oc_batch(const BatchOcDesc* D, int nprob, unsigned* queue, double move, double
 }
 
 // One cluster up to OC_CLUSTER_MAX elements, the whole grid beyond.  A call (with its host read) in
-// us, cluster / grid: 4,800 elements 54 / 73, 49,152 67 / 74, 65,536 73 / 68, 110,592 97 / 68,
-// 221,184 144 / 74: the cluster's 16 SMs run out of FP64 rate (four operations per element and
+// us, cluster / grid: 4,800 elements 40 / 57, 20,000 45 / 58, 49,152 53 / 62, 65,536 59 / 59, 110,592
+// 82 / 61, 221,184 129 / 67: the cluster's 16 SMs run out of FP64 rate (four operations per element and
 // candidate), the grid's passes cost their launches whatever the size.  The launches with host
 // reads and divisions that both replace took 356 us at 4,800, 363 at 65,536, 776 at 524,288
-// (now 96) and 2,086 at 4.2M elements (now 309).
+// (now 83) and 2,086 at 4.2M elements (now 295).
 constexpr long long OC_CLUSTER_MAX = 49152;
 
 int oc_launch(long long n, const double* rho, const double* dr, double A, double vol, double vf, double move,
@@ -948,7 +948,7 @@ int energy2_user(const Geo& g, const K2Dense& K, const KHat2<double>* box, const
 
 // ------------------------------------------------------------------ operator on user vectors, 3-D
 // K(E) u (or the element energies u_e^T K0 u_e) straight from the user's interleaved vector, FP64.
-// The walk is the one of the TMA kernel (fine_tma.cuh): 8 warps of 16 z-lanes x 2 x-columns march
+// The walk is the one of the TMA kernel (fine_tma.cuh): 4 warps of 16 z-lanes x 2 x-columns march
 // along y with one element per thread and layer, in the Walsh transform domain.  A user row (3 nz
 // doubles) has no 16-byte pitch, so planes arrive by 8-byte cp.async copies into a four-stage ring
 // (zero-filled outside the grid), each thread copying the same four positions of every plane; E and the
@@ -962,7 +962,8 @@ int energy2_user(const Geo& g, const K2Dense& K, const KHat2<double>* box, const
 // What bounds it: FP64 latency at 12 warps per SM.  An element takes 150 FP64 operations (200 without
 // the cube's block form): 45 us of the FP64 pipe at 12.8M DOF with the tiles' overlap, 37 us for the
 // bytes; it runs in 134.  Blocks of 4 warps at 168 registers, three per SM, measured best: 8 warps at
-// 128 registers 144 us (spills), four blocks 152 (spills), two 167.  The three launches it replaces
+// 128 registers 144 us (spills), four blocks 152 (spills), two 167.  (Without the block form the product
+// spills 48 bytes at 168 registers.)  The three launches it replaces
 // (user to slots, TMA product, slots to user) took 205 us.
 constexpr int U3_BX = 4, U3_NS = 4;
 constexpr int U3_NC = 2 * U3_BX, U3_NR = U3_NC + 1, U3_ROW = 51;  // element columns, node rows, doubles per row
@@ -1271,9 +1272,9 @@ static User3Tiles user3_tiles(const Geo& g, bool product) {
 }
 
 // Rows per block: the number of y-chunks that needs the fewest layers in all, counting the waves of
-// resident blocks (three per SM) and one and a half layers of start-up per block.  Up to 4,096 candidates:
-// a plan of the grid, made once with the
-// problem (made in every call, the energies of 8 x 4,000 x 8 elements took 18.8 us instead of 8.8).
+// resident blocks (three per SM) and one and a half layers of start-up per block.  Up to 4,096
+// candidates: a plan of the grid, made once with the problem (made in every call, the energies of
+// 8 x 4,000 x 8 elements took 18.8 us instead of 8.8).
 int user3_rows(const Geo& g, bool product) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
